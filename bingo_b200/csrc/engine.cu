@@ -442,30 +442,60 @@ __global__ void __launch_bounds__(kBlock) k_pair_slots(StoreView S, const unsign
 static_assert(kBlock % 32 == 0, "whole warps");
 
 // Resident 256-thread blocks per SM each walk variant is compiled for
-// (register budget 65536 / (256 * blocks)): DeepWalk and sampling 32
-// registers; PPR 40 (48 with a job table); node2vec 48 (64 with a job
-// table); the mixed-app kernel 64.
+// (register budget 65536 / (256 * blocks)).
 constexpr int walk_min_blocks(int app, bool multi) {
-  return app == APP_DEEPWALK || app == APP_SAMPLING ? 8
-         : app == APP_PPR                           ? (multi ? 5 : 6)
-         : app == APP_NODE2VEC                      ? (multi ? 4 : 5)
-                                                    : 4;
+  return app == APP_SAMPLING ? 8 : app == APP_DEEPWALK ? 5 : app == APP_PPR ? 5 : 4;
+}
+// Entries of a lane's output line (RowStage): 128 bytes, and 64 where the
+// trial scratch also takes shared memory (L1 holds the reads in flight, so
+// what lines take from it counts: node2vec and mixed tables lose 3 % at 128).
+constexpr int walk_line(int app) { return app == APP_NODE2VEC || app < 0 ? 16 : 32; }
+
+// The job of a work item: the last one that starts at or before it.
+__device__ __forceinline__ uint32_t job_of_item(const uint32_t* __restrict__ prefix, uint32_t n_jobs, uint32_t item) {
+  uint32_t lo = 0, hi = n_jobs;
+  while (hi - lo > 1) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (prefix[mid] <= item)
+      lo = mid;
+    else
+      hi = mid;
+  }
+  return lo;
 }
 
 template <int APP, bool MULTI>
 __global__ void __launch_bounds__(kBlock, walk_min_blocks(APP, MULTI))
     k_walk(WalkView W, WalkJobDev J0, const WalkJobDev* __restrict__ jobs, const uint32_t* __restrict__ prefix,
            uint32_t n_jobs, uint32_t total, uint32_t* queue, uint32_t chunk) {
-  __shared__ __align__(16) int32_t obuf[kBlock][8];
+  constexpr int kLine = walk_line(APP);
+  using Stage = RowStage<kLine>;
+  constexpr bool kRows = APP != APP_SAMPLING;                   // sampling jobs write no rows
+  constexpr bool kTrials = APP == APP_NODE2VEC || APP < 0;       // walks whose steps may take several trials
+  __shared__ int32_t obuf[kRows ? kBlock * Stage::kPitch : 1];
+  __shared__ TrialScratch trials[kTrials ? kBlock / 32 : 1];
+  __shared__ WalkJobDev one;  // the single job, where lanes index jobs
+  if (kTrials && !MULTI) {
+    if (threadIdx.x == 0) one = J0;
+    __syncthreads();
+  }
   const int lane = threadIdx.x & 31;
+  int32_t* const wbuf = obuf + (kRows ? (threadIdx.x & ~31u) * Stage::kPitch : 0);
+  int32_t* const buf = wbuf + (kRows ? lane * Stage::kPitch : 0);
   LaneWalk s;
-  RowStage o{kNoSec, 0};
   uint32_t jid = 0, moves = 0, wb = 0, we = 0;
   s.trials = 0, s.probes = 0;
+  s.i = s.j = s.cur = s.lo = s.phoff = s.phmask = s.t = 0, s.row = nullptr, s.prev = -1, s.region = 0;
   bool active = false, drained = false;
+  const uint32_t warps = gridDim.x * (kBlock / 32);
+  // A small launch's walks spread over all its warps (walks that take trials
+  // spread inside theirs).
+  const uint32_t lanes = kTrials ? 32u : min(32u, (total + warps - 1) / warps);
   for (;;) {
-    uint32_t idle = __ballot_sync(kFull, !active);
-    while (idle && !drained) {
+    uint32_t idle = drained ? 0u : __ballot_sync(kFull, !active);
+    uint32_t room = 0;
+    if (idle) room = lanes - min(lanes, 32u - __popc(idle));
+    while (idle && room && !drained) {
       if (wb >= we) {
         uint32_t base = 0;
         if (lane == 0) base = atomicAdd(queue, chunk);
@@ -477,41 +507,40 @@ __global__ void __launch_bounds__(kBlock, walk_min_blocks(APP, MULTI))
         wb = base;
         we = base + min(chunk, total - base);
       }
-      const uint32_t take = min((uint32_t)__popc(idle), we - wb);
+      const uint32_t take = min(min((uint32_t)__popc(idle), room), we - wb);
+      room -= take;
       const uint32_t rank = __popc(idle & lanemask_lt());
       if (!active && rank < take) {
         const uint32_t item = wb + rank;
         if (!MULTI) {
-          active = walk_begin<APP>(W, J0, item, s, o, obuf, moves);
+          active = walk_begin<APP, kLine>(W, J0, item, s, buf, moves);
         } else {
-          uint32_t lo = 0, hi = n_jobs;
-          while (hi - lo > 1) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (prefix[mid] <= item)
-              lo = mid;
-            else
-              hi = mid;
-          }
-          jid = lo;
-          if (APP >= 0)
-            active = walk_begin<APP>(W, jobs[lo], item - prefix[lo], s, o, obuf, moves);
-          else
-            active = begin_any(W, jobs[lo], item - prefix[lo], s, o, obuf, moves);
+          jid = job_of_item(prefix, n_jobs, item);
+          active = walk_begin<APP, kLine>(W, jobs[jid], item - prefix[jid], s, buf, moves);
         }
       }
       wb += take;
       idle = __ballot_sync(kFull, !active);
     }
-    if (!__any_sync(kFull, active)) break;
-    if (active) {
-      constexpr int A = APP == APP_SAMPLING ? APP_DEEPWALK : APP;
-      if (!MULTI)
-        active = walk_advance<A>(W, J0, s, o, obuf, moves);
-      else if (APP >= 0)
-        active = walk_advance<A>(W, jobs[jid], s, o, obuf, moves);
-      else
-        active = advance_any(W, jobs[jid], s, o, obuf, moves);
+    if (!__any_sync(kFull, active)) {
+      if (drained) break;
+      continue;
     }
+    if (!kRows) continue;
+    constexpr int A = APP == APP_SAMPLING ? APP_DEEPWALK : APP;
+    const WalkJobDev& J = MULTI ? jobs[jid] : J0;
+    bool out = false, end = false;
+    uint32_t pos = 0;
+    Proposal p{-1, false, false, 0, 0};
+    if (kTrials)
+      p = warp_propose<A>(W, MULTI ? jobs : &one, jid, s, active, trials[threadIdx.x / 32]);
+    else if (active)
+      p = walk_propose<A>(W, J, s);
+    if (active && p.ok) {
+      active = walk_commit<A, kLine>(J, s, p, buf, moves, out, pos);
+      end = !active;
+    }
+    Stage::flush(wbuf, out, end, s, pos, J.L);
   }
   add_steps(W, moves);
   add_n2v(W, s);
@@ -543,18 +572,17 @@ unsigned walk_blocks_per_sm() {
 }
 
 // Default launch shape of each walk kernel (the knobs' value 0), measured on
-// B200 with fixed graphs, launches interleaved: resident 256-thread blocks
-// per SM (0 = the occupancy limit) and walks a warp claims per refill.
-// DeepWalk (R-MAT scale 20, 16 M edges, log-uniform weights): 26.3 G
-// steps/s at 4 blocks and 8 walks against 21.7 G at its 8-block occupancy
-// limit and 32 (more resident warps issue more concurrent random reads than
-// DRAM turns into throughput; 2 blocks: 23.0 G). PPR: 11.3 G at 4 blocks and
-// 32 against 11.0 G at 6. node2vec (R-MAT scale 22, Zipf weights) and the
-// mixed-app table (R-MAT scale 22, 16 mixed jobs) run best at their
-// occupancy limits (5 and 4 blocks) with 32. One-hop sampling (one step per
-// item) keeps the occupancy limit and 32.
+// B200, launches interleaved: resident 256-thread blocks per SM (0 = the
+// occupancy limit) and walks a warp claims per refill. DeepWalk and PPR run
+// 4 blocks: past that the concurrent random reads only queue (DeepWalk, R-MAT
+// 20, at 4 and 8 blocks: 26.3 and 21.7 G steps/s). Claims: what a warp holds
+// unstarted waits for its lanes, which is worst for long walks: 16 jobs of
+// all apps on R-MAT 20 (1.1 M walks) take 3.3 ms at 32 walks per claim, 2.2
+// at 8 and 1.95 at 4; DeepWalk (1 M walks) 1080 us at 8, 1093 at 16. A launch
+// that fits its lanes claims each warp's share at once. One-hop sampling (one
+// step per item) keeps the occupancy limit and 32.
 constexpr unsigned walk_default_bps(int app) { return app == APP_DEEPWALK || app == APP_PPR ? 4 : 0; }
-constexpr uint32_t walk_default_chunk(int app) { return app == APP_DEEPWALK ? 8 : 32; }
+constexpr uint32_t walk_default_chunk(int app) { return app == APP_NODE2VEC || app < 0 ? 4 : app == APP_DEEPWALK ? 8 : 32; }
 
 // Blocks per SM for a walk launch of `app` (-1: mixed table): the tuned or
 // default figure, capped by occupancy.
@@ -562,39 +590,78 @@ unsigned walk_bps(unsigned occ, const Tuning& t, int app) {
   const unsigned want = t.walk_blocks_per_sm ? t.walk_blocks_per_sm : walk_default_bps(app);
   return want ? std::max(1u, std::min(occ, want)) : occ;
 }
-uint32_t walk_chunk_of(const Tuning& t, int app) { return t.walk_chunk ? t.walk_chunk : walk_default_chunk(app); }
+uint32_t walk_chunk_of(const Tuning& t, int app, uint32_t total, unsigned grid) {
+  if (t.walk_chunk) return t.walk_chunk;
+  const uint32_t warps = grid * (kBlock / 32);
+  const bool one_fill = app != APP_NODE2VEC && app >= 0 && total <= 32ull * warps;  // every warp claims its share at once
+  return one_fill ? (total + warps - 1) / warps : walk_default_chunk(app);
+}
+
+// Blocks of a walk launch: one resident wave at most, and at least
+// walk_per_block walks per block: half-full warps on twice the SMs finish
+// sooner (16,384 DeepWalk walks of 80 on R-MAT 14: 80 us at 256 walks per
+// block, 73 at 128), and walks that take trials use the idle lanes.
+constexpr unsigned walk_per_block(int app) { return app == APP_NODE2VEC || app < 0 ? 64 : app == APP_SAMPLING ? 256 : 128; }
+template <int APP, bool MULTI>
+unsigned walk_grid(unsigned long long total, const Tuning& t) {
+  return grid_for(total, walk_per_block(APP), walk_bps(walk_blocks_per_sm<APP, MULTI>(), t, APP));
+}
+
+template <int APP, bool MULTI>
+void launch_walk(cudaStream_t st, const WalkView& W, const WalkJobDev& J0, const WalkJobDev* jobs,
+                 const uint32_t* prefix, uint32_t n_jobs, uint32_t total, uint32_t* queue, const Tuning& t) {
+  const unsigned grid = walk_grid<APP, MULTI>(total, t);
+  k_walk<APP, MULTI><<<grid, kBlock, 0, st>>>(W, J0, jobs, prefix, n_jobs, total, queue,
+                                              walk_chunk_of(t, APP, total, grid));
+}
 
 // Launches the persistent walk kernel for a device job table whose jobs all
 // have app `app` (or any app when app < 0).
 void launch_walk_table(cudaStream_t st, int app, const WalkView& W, const WalkJobDev& J0, const WalkJobDev* jobs,
                        const uint32_t* prefix, uint32_t n_jobs, uint32_t total, uint32_t* queue, const Tuning& t) {
-  const uint32_t c = walk_chunk_of(t, app);
-  switch (app) {
-    case APP_DEEPWALK:
-      k_walk<APP_DEEPWALK, true>
-          <<<grid_for(total, kBlock, walk_bps(walk_blocks_per_sm<APP_DEEPWALK, true>(), t, APP_DEEPWALK)), kBlock, 0, st>>>(
-              W, J0, jobs, prefix, n_jobs, total, queue, c);
-      break;
-    case APP_NODE2VEC:
-      k_walk<APP_NODE2VEC, true>
-          <<<grid_for(total, kBlock, walk_bps(walk_blocks_per_sm<APP_NODE2VEC, true>(), t, APP_NODE2VEC)), kBlock, 0, st>>>(
-              W, J0, jobs, prefix, n_jobs, total, queue, c);
-      break;
-    case APP_PPR:
-      k_walk<APP_PPR, true><<<grid_for(total, kBlock, walk_bps(walk_blocks_per_sm<APP_PPR, true>(), t, APP_PPR)), kBlock, 0, st>>>(
-          W, J0, jobs, prefix, n_jobs, total, queue, c);
-      break;
-    case APP_SAMPLING:
-      k_walk<APP_SAMPLING, true>
-          <<<grid_for(total, kBlock, walk_bps(walk_blocks_per_sm<APP_SAMPLING, true>(), t, APP_SAMPLING)), kBlock, 0, st>>>(
-              W, J0, jobs, prefix, n_jobs, total, queue, c);
-      break;
-    default:
-      k_walk<-1, true><<<grid_for(total, kBlock, walk_bps(walk_blocks_per_sm<-1, true>(), t, -1)), kBlock, 0, st>>>(
-          W, J0, jobs, prefix, n_jobs, total, queue, c);
-      break;
-  }
+  auto* go = app == APP_DEEPWALK   ? launch_walk<APP_DEEPWALK, true>
+             : app == APP_NODE2VEC ? launch_walk<APP_NODE2VEC, true>
+             : app == APP_PPR      ? launch_walk<APP_PPR, true>
+             : app == APP_SAMPLING ? launch_walk<APP_SAMPLING, true>
+                                   : launch_walk<-1, true>;
+  go(st, W, J0, jobs, prefix, n_jobs, total, queue, t);
   cuda_check(cudaGetLastError(), "walk launch");
+}
+
+// One job's walks (the plain form).
+void launch_walk_job(cudaStream_t st, const WalkView& W, const WalkJobDev& J, uint32_t* queue, const Tuning& t) {
+  auto* go = J.app == APP_DEEPWALK   ? launch_walk<APP_DEEPWALK, false>
+             : J.app == APP_NODE2VEC ? launch_walk<APP_NODE2VEC, false>
+             : J.app == APP_PPR      ? launch_walk<APP_PPR, false>
+                                     : launch_walk<APP_SAMPLING, false>;
+  go(st, W, J, nullptr, nullptr, 0, (uint32_t)J.n, queue, t);
+  cuda_check(cudaGetLastError(), "walk launch");
+}
+
+// Shared memory against L1: a read in flight holds an L1 line, so each walk
+// kernel asks for no more shared memory than its resident blocks use (1 M
+// DeepWalk walks with 128-byte lines: 1968 us with the default split, 1080
+// with this one).
+template <int APP, bool MULTI>
+void walk_carveout(unsigned blocks) {
+  cudaFuncAttributes fa;
+  cuda_check(cudaFuncGetAttributes(&fa, k_walk<APP, MULTI>), "walk kernel attributes");
+  const unsigned kb = (unsigned)((blocks * (fa.sharedSizeBytes + 1024) + 1023) / 1024);
+  cuda_check(cudaFuncSetAttribute(k_walk<APP, MULTI>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                  (int)std::min(100u, (kb * 100 + 227) / 228)),
+             "walk kernel carve-out");
+}
+
+// All walk kernels, once per device (the current one).
+void walk_carveouts(int device) {
+  static std::mutex mu;
+  static std::vector<int> done;
+  std::lock_guard<std::mutex> lock(mu);
+  if (std::find(done.begin(), done.end(), device) != done.end()) return;
+  walk_carveout<APP_DEEPWALK, false>(4), walk_carveout<APP_DEEPWALK, true>(4);
+  walk_carveout<APP_PPR, false>(4), walk_carveout<APP_PPR, true>(4);
+  walk_carveout<APP_NODE2VEC, false>(4), walk_carveout<APP_NODE2VEC, true>(4), walk_carveout<-1, true>(4);
+  done.push_back(device);
 }
 
 // A job table for one persistent launch: jobs of one app (or all apps).
@@ -747,6 +814,7 @@ Engine::Engine(const bingo_config& cfg) : cfg_(cfg) {
              "cudaHostAlloc(plan)");
   cuda_check(cudaHostGetDevicePointer((void**)&d_plan_, (void*)h_plan_, 0), "plan mapping");
   cuda_check(cudaEventCreateWithFlags(&slots_ev_, cudaEventDisableTiming), "cudaEventCreate");
+  walk_carveouts(cfg.device);
 }
 
 Engine::~Engine() {
@@ -1482,16 +1550,6 @@ void Engine::walk(const bingo_walk_job* jobs, uint32_t n_jobs, uint32_t mode) {
       throw Error(BINGO_ERR_INVALID_ARGUMENT, "device output must be 32-byte aligned");
   }
   const WalkView W = wview();
-  auto launch = [&](auto kern, unsigned occ, const WalkJobDev& J0, const WalkJobDev* jb, const uint32_t* pf,
-                    uint32_t nj, uint32_t tot, uint32_t* qq) {
-    cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3(grid_for(tot, kBlock, walk_bps(occ, tuning_, J0.app)));
-    lc.blockDim = dim3(kBlock);
-    lc.stream = stream_;
-    cuda_check(cudaLaunchKernelEx(&lc, kern, W, J0, jb, pf, nj, tot, qq, walk_chunk_of(tuning_, J0.app)),
-               "walk launch");
-    ++launches_;
-  };
   queue_.ensure(4 * std::max<uint32_t>(n_jobs, 4), "walk queue");
   uint32_t* q = queue_.as<uint32_t>();
   if (mode == BINGO_WALK_PLAIN) {
@@ -1499,25 +1557,8 @@ void Engine::walk(const bingo_walk_job* jobs, uint32_t n_jobs, uint32_t mode) {
     cuda_check(cudaMemsetAsync(q, 0, 4 * n_jobs, stream_), "queue reset");
     for (uint32_t j = 0; j < n_jobs; ++j) {
       if (!dj[j].n) continue;
-      const uint32_t nw = (uint32_t)dj[j].n;
-      switch (dj[j].app) {
-        case APP_DEEPWALK:
-          launch(k_walk<APP_DEEPWALK, false>, walk_blocks_per_sm<APP_DEEPWALK, false>(), dj[j], nullptr,
-                 nullptr, 0, nw, q + j);
-          break;
-        case APP_NODE2VEC:
-          launch(k_walk<APP_NODE2VEC, false>, walk_blocks_per_sm<APP_NODE2VEC, false>(), dj[j], nullptr,
-                 nullptr, 0, nw, q + j);
-          break;
-        case APP_PPR:
-          launch(k_walk<APP_PPR, false>, walk_blocks_per_sm<APP_PPR, false>(), dj[j], nullptr, nullptr, 0,
-                 nw, q + j);
-          break;
-        default:
-          launch(k_walk<APP_SAMPLING, false>, walk_blocks_per_sm<APP_SAMPLING, false>(), dj[j], nullptr,
-                 nullptr, 0, nw, q + j);
-          break;
-      }
+      launch_walk_job(stream_, W, dj[j], q + j, tuning_);
+      ++launches_;
     }
   } else if (prefix[n_jobs]) {
     // One persistent launch per app present (or one mixed launch).
@@ -1933,9 +1974,8 @@ void Engine::walk_noalloc(const bingo_walk_job* jobs, uint32_t n_jobs) {
   cuda_check(cudaGetLastError(), "no-alloc job staging");
   ++launches_;
   const WalkView W = wview();
-  k_walk<-1, true><<<grid_for(total, kBlock, walk_bps(walk_blocks_per_sm<-1, true>(), tuning_, -1)), kBlock, 0, stream_>>>(
-      W, dj[0], scratch->jobs, scratch->prefix, n_jobs, (uint32_t)total, &scratch->queue, walk_chunk_of(tuning_, -1));
-  cuda_check(cudaGetLastError(), "no-alloc walk launch");
+  launch_walk_table(stream_, -1, W, dj[0], scratch->jobs, scratch->prefix, n_jobs, (uint32_t)total, &scratch->queue,
+                    tuning_);
   ++launches_;
   finish_call();
 }

@@ -40,6 +40,7 @@ namespace bingo {
 namespace {
 
 constexpr int kServeBlock = 256;
+constexpr int kServeLine = 16;  // output line entries: with the job copies, under 48 KB of shared memory per block
 constexpr uint32_t kPollSteps = 8;
 constexpr uint32_t kSpinPasses = 20000;  // scheduler passes polled without sleeping
 
@@ -83,20 +84,25 @@ __device__ __forceinline__ uint32_t claim_walks(const WalkJobDev* __restrict__ j
 __global__ void __launch_bounds__(kServeBlock, 4)
     k_serve(WalkView W, const WalkJobDev* __restrict__ jobs, const ServeCtl* ctl, ServeDevState* st,
             volatile unsigned long long* done_seq, volatile unsigned long long* err_word, uint32_t idle_us) {
-  __shared__ __align__(16) int32_t obuf[kServeBlock][8];
+  using Stage = RowStage<kServeLine>;
+  __shared__ int32_t obuf[kServeBlock * Stage::kPitch];
   __shared__ __align__(16) WalkJobDev jc[kServeBlock];
   const int lane = threadIdx.x & 31;
   WalkJobDev& J = jc[threadIdx.x];
+  int32_t* const wbuf = obuf + (threadIdx.x & ~31u) * Stage::kPitch;
+  const uint32_t mine = lane * Stage::kPitch;
+  __shared__ TrialScratch trials[kServeBlock / 32];
+  const WalkJobDev* const wjc = jc + (threadIdx.x & ~31u);  // this warp's job copies, by lane
   LaneWalk s;
-  RowStage o{kNoSec, 0};
   uint32_t moves = 0, jseq = 0, nap = 256, poll_in = 0;
   s.trials = 0, s.probes = 0;
+  s.i = s.j = s.cur = s.lo = s.phoff = s.phmask = s.t = 0, s.row = nullptr, s.prev = -1, s.region = 0;
   unsigned long long idle_ns = 0;
   uint32_t wj = 0, wb = 0, we = 0;  // this warp's claimed range: walks [wb, we) of job wj
   bool active = false;
 
   auto finish = [&]() {
-    __threadfence();  // this lane's row writes before the completion count
+    __threadfence();  // this walk's row writes before the completion count
     const uint32_t slot = jseq & (kServeMaxJobs - 1);
     if (atomicAdd(&st->done[slot], 1u) + 1 == (uint32_t)J.n) {
       __threadfence_system();
@@ -139,7 +145,7 @@ __global__ void __launch_bounds__(kServeBlock, 4)
         int4* dst = reinterpret_cast<int4*>(&J);
 #pragma unroll
         for (int t = 0; t < (int)(sizeof(WalkJobDev) / 16); ++t) dst[t] = __ldcg(src + t);
-        active = begin_any(W, J, wb + rank, s, o, obuf, moves);
+        active = walk_begin<-1, kServeLine>(W, J, wb + rank, s, wbuf + mine, moves);
         if (!active) finish();
       }
       wb += take;
@@ -168,9 +174,18 @@ __global__ void __launch_bounds__(kServeBlock, 4)
     }
     nap = 256;
     idle_ns = 0;
-    if (active) {
-      active = advance_any(W, J, s, o, obuf, moves);
-      if (!active) finish();
+    bool out = false, end = false;
+    uint32_t pos = 0;
+    const Proposal p = warp_propose<-1>(W, wjc, (uint32_t)lane, s, active, trials[threadIdx.x / 32]);
+    if (active && p.ok) {
+      active = walk_commit<-1, kServeLine>(J, s, p, wbuf + mine, moves, out, pos);
+      end = !active;
+    }
+    Stage::flush(wbuf, out, end, s, pos, out ? J.L : 0u);
+    if (__any_sync(kFull, end)) {
+      __threadfence();  // lanes wrote one another's rows: each orders its own stores before the counts below
+      __syncwarp();
+      if (end) finish();
     }
   }
   add_steps(W, moves);

@@ -143,27 +143,38 @@ __device__ __forceinline__ void hash_sub(HashEntry* tab, uint32_t hmask, uint32_
   }
 }
 
-// Index of v's entry, or -1.
-__device__ __forceinline__ int hash_find(const HashEntry* tab, uint32_t hmask, uint32_t v) {
-  uint32_t h = mix32(v) & hmask;
-  for (uint32_t probe = 0; probe <= hmask; ++probe) {
+// Lookup of v in two parts, so that its reads can be under way beside others:
+// hash_peek loads the keys that the first sector of v's probe sequence holds
+// (one or two), and hash_settle gives the index of v's entry, or -1.
+struct HashPeek {
+  uint32_t h;
+  int key0, key1;
+};
+__device__ __forceinline__ void hash_peek(HashPeek& p, const HashEntry* tab, uint32_t hmask, uint32_t v) {
+  p.h = mix32(v) & hmask;
+  p.key0 = __ldg(&tab[p.h].key);
+  p.key1 = __ldg(&tab[(p.h | 1u) & hmask].key);
+}
+__device__ __forceinline__ int hash_settle(const HashPeek& p, const HashEntry* tab, uint32_t hmask, uint32_t v) {
+  if (p.key0 == (int)v) return (int)p.h;
+  if (p.key0 == kEmptyKey) return -1;
+  uint32_t h = (p.h | 1u) & hmask;
+  if (p.key1 == (int)v) return (int)h;
+  if (p.key1 == kEmptyKey) return -1;
+  for (uint32_t probe = 1; probe <= hmask; ++probe) {
+    h = (h + 1) & hmask;
     const int k = __ldg(&tab[h].key);
     if (k == (int)v) return (int)h;
     if (k == kEmptyKey) return -1;
-    h = (h + 1) & hmask;
   }
   return -1;
 }
 
 __device__ __forceinline__ bool hash_has(const HashEntry* tab, uint32_t hmask, uint32_t v) {
-  const int h = hash_find(tab, hmask, v);
+  HashPeek p;
+  hash_peek(p, tab, hmask, v);
+  const int h = hash_settle(p, tab, hmask, v);
   return h >= 0 && __ldg(&tab[h].cnt) > 0;
-}
-
-// Live weight sum of the edges to v (0 when there are none).
-__device__ __forceinline__ unsigned long long hash_weight(const HashEntry* tab, uint32_t hmask, uint32_t v) {
-  const int h = hash_find(tab, hmask, v);
-  return h >= 0 && __ldg(&tab[h].cnt) > 0 ? __ldg(&tab[h].wsum) : 0ull;
 }
 
 // ---------------------------------------------------------------------------

@@ -61,28 +61,46 @@ __device__ __forceinline__ VertexRec load_vrec(const WalkView& W, uint32_t u) {
   return VertexRec{r.x, r.y, r.z, r.w};
 }
 
-// Weighted neighbour draw at a vertex with R.m > 0: slot = mulhi(x, m),
-// r = mulhi64(y:z, T), group = r < thr ? own : alias, member = mulhi(w, cnt)
-// (a one-member group carries its member in the slot: mulhi(w, 1) = 0).
-__device__ __forceinline__ uint32_t sample_at(const WalkView& W, const VertexRec& R, const Rand4& r) {
+// Weighted neighbour draw at a vertex with m > 0 alias slots from aoff: slot =
+// mulhi(x, m), r = mulhi64(y:z, T), group = r < thr ? own : alias, member =
+// mulhi(w, cnt) (a one-member group carries its member in the slot:
+// mulhi(w, 1) = 0). In three parts, so that a lane can have several draws'
+// reads in flight.
+struct SlotRead {
+  unsigned long long thr, T, own_rc, alt_rc;
+};
+__device__ __forceinline__ void slot_load(SlotRead& q, const WalkView& W, uint32_t aoff, uint32_t m, const Rand4& r) {
   // The whole 32-byte slot in one 256-bit read-only load (one L1 / L2
   // request instead of two 16-byte ones; slots are 32-byte aligned and no
   // kernel writes the store while walks run).
-  const AliasRec* a = W.alias + R.aoff + mulhi32(r.x, R.m);
-  unsigned long long thr, T, own_rc, alt_rc;
-  asm("ld.global.nc.v4.u64 {%0, %1, %2, %3}, [%4];" : "=l"(thr), "=l"(T), "=l"(own_rc), "=l"(alt_rc) : "l"(a));
-  const unsigned long long d = mulhi64(((unsigned long long)r.y << 32) | r.z, T);
-  const unsigned long long rc = d < thr ? own_rc : alt_rc;  // ref | count word << 32
+  const AliasRec* a = W.alias + aoff + mulhi32(r.x, m);
+  asm("ld.global.nc.v4.u64 {%0, %1, %2, %3}, [%4];"
+      : "=l"(q.thr), "=l"(q.T), "=l"(q.own_rc), "=l"(q.alt_rc)
+      : "l"(a));
+}
+// The drawn group: ref | count word << 32.
+__device__ __forceinline__ unsigned long long slot_pick(const SlotRead& q, const Rand4& r) {
+  const unsigned long long d = mulhi64(((unsigned long long)r.y << 32) | r.z, q.T);
+  return d < q.thr ? q.own_rc : q.alt_rc;
+}
+__device__ __forceinline__ uint32_t member_load(const WalkView& W, unsigned long long rc, const Rand4& r) {
   const uint32_t ref = (uint32_t)rc, cw = (uint32_t)(rc >> 32);
   if (cw & kInlineGroup) return ref;  // one member, carried in the slot
   return __ldg(W.gv + (size_t)ref * 4 + mulhi32(r.w, cw));
 }
-
+__device__ __forceinline__ uint32_t sample_at(const WalkView& W, uint32_t aoff, uint32_t m, const Rand4& r) {
+  SlotRead q;
+  slot_load(q, W, aoff, m, r);
+  return member_load(W, slot_pick(q, r), r);
+}
 
 // ---------------------------------------------------------------------------
 // Step-at-a-time walks for the persistent kernels: a lane advances its walk
 // one step per iteration and pulls a new walk as soon as its walk ends, so
-// dead-ended and early-stopped walks do not idle their warp.
+// dead-ended and early-stopped walks do not idle their warp. An iteration is
+// warp-converged: every lane proposes its next vertex (walk_propose), commits
+// it (walk_commit), and the warp writes out finished output lines together
+// (RowStage::flush).
 //
 // Counters: step j of walk i in job `job` draws Philox block
 // (i, j, trial, job) under key seed. DeepWalk uses trial 0; PPR samples with
@@ -90,93 +108,81 @@ __device__ __forceinline__ uint32_t sample_at(const WalkView& W, const VertexRec
 // and accepts with trial 2t + 1 (t = 0, 1, ...; the first step is
 // first-order and takes trial 0). Row position j holds the j-th move; a walk
 // that reaches a vertex without out-edges writes -1 there and pads the rest.
-//
-// Row output goes through an 8-entry (one 32-byte sector) staging buffer per
-// lane in shared memory: a lane writes its row a whole sector at a time with
-// streaming (evict-first) stores, so the write-once walk output neither
-// lands in L2 as partial sectors nor evicts graph data.
-struct RowStage {
-  uint32_t sec;   // index of the buffered 32-byte sector within the job output; kNoSec: empty
-  uint32_t lohi;  // valid entries [lo, hi) of the sector: lo | hi << 8
-};
-constexpr uint32_t kNoSec = 0xffffffffu;
-
-// This lane's 8 staging entries (16-byte aligned, blockDim.x rows of 8).
-__device__ __forceinline__ int32_t* stage_buf(int32_t (*obuf)[8]) { return obuf[threadIdx.x]; }
-
-__device__ __forceinline__ void stage_flush(RowStage& o, int32_t* out, int32_t (*obuf)[8]) {
-  if (o.sec == kNoSec) return;
-  const int32_t* buf = stage_buf(obuf);
-  int32_t* sec = out + (size_t)o.sec * 8;
-  const uint32_t lo = o.lohi & 0xff, hi = o.lohi >> 8;
-  if (lo == 0 && hi == 8) {
-    const int4* b = reinterpret_cast<const int4*>(buf);
-    __stcs(reinterpret_cast<int4*>(sec), b[0]);
-    __stcs(reinterpret_cast<int4*>(sec) + 1, b[1]);
-  } else {
-    for (uint32_t t = lo; t < hi; ++t) __stcs(sec + t, buf[t]);
-  }
-  o.sec = kNoSec;
-}
-
-// Writes v to out[g] through the stage; a row's positions arrive in
-// non-decreasing order (PPR tail mode rewrites the last one). Job outputs are
-// 32-byte aligned, so sectors are counted from out.
-__device__ __forceinline__ void stage_put(RowStage& o, int32_t* out, int32_t (*obuf)[8], unsigned long long g,
-                                          int32_t v) {
-  const uint32_t sec = (uint32_t)(g >> 3), t = (uint32_t)(g & 7);
-  if (sec != o.sec) {
-    stage_flush(o, out, obuf);
-    o.sec = sec;
-    o.lohi = t | (t << 8);
-  }
-  stage_buf(obuf)[t] = v;
-  if (t + 1 > (o.lohi >> 8)) o.lohi = (o.lohi & 0xff) | ((t + 1) << 8);
-}
-
-// Pads out[g, g_end) with -1: the open sector through the stage, then whole
-// sectors with two 16-byte streaming stores each.
-__device__ __forceinline__ void stage_pad(RowStage& o, int32_t* out, int32_t (*obuf)[8], unsigned long long g,
-                                          unsigned long long g_end) {
-  for (; g < g_end && (g & 7); ++g) stage_put(o, out, obuf, g, -1);
-  stage_flush(o, out, obuf);
-  const int4 m1 = make_int4(-1, -1, -1, -1);
-  for (; g + 8 <= g_end; g += 8) {
-    __stcs(reinterpret_cast<int4*>(out + g), m1);
-    __stcs(reinterpret_cast<int4*>(out + g) + 1, m1);
-  }
-  for (; g < g_end; ++g) __stcs(out + g, -1);
-}
-
-// node2vec trials a lane runs before it yields the rest of the step to the
-// next call (the rest of its warp moves on meanwhile).
-constexpr uint32_t kNode2vecTrialsPerCall = 3;
 
 struct LaneWalk {
   uint32_t i;      // walk index within its job
   uint32_t j;      // step being produced
   uint32_t cur;    // current vertex
-  uint32_t pos;    // last row position written
+  uint32_t lo;     // first entry of the open output line that belongs to this row
+  int32_t* row;    // the walk's output row
   int32_t prev;    // previous vertex (node2vec), -1 before the first move
   uint32_t phoff;  // previous vertex's adjacency index (node2vec)
   uint32_t phmask;
+  uint32_t t;       // node2vec: first trial not yet drawn of the step in progress (0 = a new step)
   uint32_t trials;  // node2vec proposals drawn by this lane (kept across its walks)
   uint32_t probes;  // node2vec adjacency-index lookups by this lane
-  uint32_t t;       // node2vec: trial of the step in progress (0 = a new step)
   unsigned long long region;  // node2vec: return-region threshold of the step in progress
 };
 
+// Output lines. A lane collects its row a LINE (entries) at a time in shared
+// memory; the warp then writes the line with one coalesced streaming store,
+// and the end of a finished row with its -1 padding the same way. Walks are
+// bound by random DRAM accesses and a row write of one 32-byte sector costs
+// DRAM about as much as a read of one (R-MAT 20, 1 M walks x 80: 1138 us with
+// 32-byte writes, 998 us with none): lines of 128 bytes are a quarter of the
+// accesses. Lines are those of the address space, so a row may start and end
+// inside one (entries before `lo` and past the row's end are not touched).
+template <int LINE>
+struct RowStage {
+  static_assert(LINE == 8 || LINE == 16 || LINE == 32, "an entry per lane at most");
+  // One lane's entries; the odd pitch spreads lanes at equal positions over the banks.
+  static constexpr uint32_t kPitch = LINE + 1;
+
+  static __device__ __forceinline__ uint32_t slot(const int32_t* p) {
+    return (uint32_t)(reinterpret_cast<uintptr_t>(p) >> 2) & (LINE - 1);
+  }
+
+  // Every lane whose `out` is set writes its open line's entries [lo, last]
+  // (last = slot of row position `pos`) and, when `end` (the row is
+  // finished), -1 from pos + 1 to the row's end. Called by the whole warp;
+  // `buf` is the warp's entries, lane l's at buf + l x kPitch.
+  static __device__ __forceinline__ void flush(const int32_t* buf, bool out, bool end, LaneWalk& s, uint32_t pos,
+                                               uint32_t L) {
+    uint32_t todo = __ballot_sync(kFull, out);
+    if (!todo) return;
+    __syncwarp();  // the entries are in shared memory
+    const uint32_t lane = threadIdx.x & 31;
+    const int32_t* e = s.row + pos;
+    const uint32_t last = slot(e);
+    const unsigned long long line = reinterpret_cast<unsigned long long>(e - last);
+    const uint32_t stop = end ? last + (L - pos) : last + 1;  // first entry after this write, from the line's start
+    const uint32_t pack = s.lo | (last << 8);
+    do {
+      const int src = __ffs(todo) - 1;
+      todo &= todo - 1;
+      int32_t* const base = reinterpret_cast<int32_t*>(__shfl_sync(kFull, line, src));
+      const uint32_t pk = __shfl_sync(kFull, pack, src), n = __shfl_sync(kFull, stop, src);
+      const uint32_t lo = pk & 0xff, hi = pk >> 8;
+      if (lane >= lo && lane < n) __stcs(base + lane, lane <= hi ? buf[src * kPitch + lane] : -1);
+      for (uint32_t x = lane + 32; x < n; x += 32) __stcs(base + x, -1);
+    } while (todo);
+    if (out) s.lo = 0;
+    __syncwarp();  // the entries may be overwritten
+  }
+};
+
 // Starts walk i; returns true if it still has steps to produce. Sampling jobs
-// complete here.
-template <int APP>
+// and rows of one position complete here. `buf`: this lane's line entries.
+template <int APP, int LINE>
 __device__ __forceinline__ bool walk_begin(const WalkView& W, const WalkJobDev& J, uint32_t i, LaneWalk& s,
-                                           RowStage& o, int32_t (*obuf)[8], uint32_t& moves) {
+                                           int32_t* buf, uint32_t& moves) {
   const uint32_t start = J.starts ? J.starts[i] : J.first + i;
-  if (APP == APP_SAMPLING) {
+  const int app = APP >= 0 ? APP : J.app;
+  if (app == APP_SAMPLING) {
     int32_t x = -1;
     if (start < W.n) {
       const VertexRec R = load_vrec(W, start);
-      if (R.m) x = (int32_t)sample_at(W, R, philox(i, 1, 0, J.job, J.k0, J.k1));
+      if (R.m) x = (int32_t)sample_at(W, R.aoff, R.m, philox(i, 1, 0, J.job, J.k0, J.k1));
     } else {
       set_err(W.err, E_RANGE);
     }
@@ -186,129 +192,232 @@ __device__ __forceinline__ bool walk_begin(const WalkView& W, const WalkJobDev& 
   }
   const uint32_t L = J.L;
   if (L == 0) return false;
-  const unsigned long long g0 = (unsigned long long)i * L;
+  s.row = J.out + (unsigned long long)i * L;
   if (start >= W.n) {
     set_err(W.err, E_RANGE);
-    stage_pad(o, J.out, obuf, g0, g0 + L);
+    for (uint32_t p = 0; p < L; ++p) __stcs(s.row + p, -1);
     return false;
   }
-  stage_put(o, J.out, obuf, g0, (int32_t)start);
+  const bool tail = app == APP_PPR && (J.flags & kWalkPprTail);
+  const uint32_t first = RowStage<LINE>::slot(s.row);
+  if (first == LINE - 1 || (L == 1 && !tail)) {  // the line ends here (or the row does): nothing to collect
+    __stcs(s.row, (int32_t)start);
+    s.lo = 0;
+    if (L == 1) {
+      if (!tail) return false;
+      s.lo = first;  // a tail row of one position rewrites this entry
+    }
+  } else {
+    buf[first] = (int32_t)start;
+    s.lo = first;
+  }
   s.i = i;
   s.j = 1;
   s.cur = start;
-  s.pos = 0;
   s.prev = -1;
   s.t = 0;
-  const bool tail = APP == APP_PPR && (J.flags & kWalkPprTail);
-  if (L > 1 || tail) return true;
-  stage_flush(o, J.out, obuf);
-  return false;
+  return true;
 }
 
-// Produces one step; returns false when the walk has ended (row padded and
-// flushed).
+// What a lane drew for the step in progress.
+struct Proposal {
+  int32_t x;             // the next vertex; -1: a dead end
+  bool ok;               // node2vec: a trial was accepted (true for the other apps)
+  bool stop;             // PPR: the walk ends after this move
+  uint32_t hoff, hmask;  // the current vertex's adjacency index (node2vec)
+};
+
+// Draws the next vertex of a first-order walk (DeepWalk, PPR). The Philox
+// blocks depend on no load: they are drawn while the vertex record is on its
+// way (R-MAT 14, 16,384 walks x 80: 85 -> 79 us).
 template <int APP>
-__device__ __forceinline__ bool walk_advance(const WalkView& W, const WalkJobDev& J, LaneWalk& s, RowStage& o,
-                                             int32_t (*obuf)[8], uint32_t& moves) {
-  const uint32_t L = J.L;
-  const bool tail = APP == APP_PPR && (J.flags & kWalkPprTail);
-  s.pos = s.j < L ? s.j : L - 1;
-  const unsigned long long g0 = (unsigned long long)s.i * L;
+__device__ __forceinline__ Proposal walk_propose(const WalkView& W, const WalkJobDev& J, const LaneWalk& s) {
   const VertexRec R = load_vrec(W, s.cur);
-  bool done = false;
-  if (!R.m) {
-    stage_put(o, J.out, obuf, g0 + s.pos, -1);
-    done = true;
-  } else {
-    uint32_t x;
-    if (APP == APP_NODE2VEC && s.prev >= 0) {
-      // One trial per call: a rejected lane keeps its step and retries on the
-      // next call while the other lanes of its warp go on, so the lanes of a
-      // warp stay on the same instruction path (the trial count per step
-      // varies from lane to lane). Trial t reads the same Philox blocks as in
-      // a loop, so the walk is unchanged.
-      if (s.t == 0) {
-        // Return region: when 1/p exceeds the envelope max(1, 1/q), the
-        // excess mass (ret_excess x w(cur -> prev)) returns to prev directly,
-        // with probability D / (T + D) per trial (word y of the acceptance
-        // block).
-        s.region = 0;
-        if (J.ret_excess > 0.0) {
-          const unsigned long long wp = hash_weight(W.hash + R.hoff, R.hmask, (uint32_t)s.prev);
-          ++s.probes;
-          if (wp) {
-            const double T = (double)__ldg(&W.alias[R.aoff].T);
-            const double D = __dmul_rn(J.ret_excess, (double)wp);
-            s.region = prob_threshold_dev(__ddiv_rn(D, __dadd_rn(T, D)));
-          }
-        }
-      }
-      // Otherwise accept a proposal x with probability weight(class(x)) /
-      // envelope. The adjacency probe is skipped when the acceptance draw is
-      // below both the in- and out-class thresholds (the outcome is then the
-      // same for every class x can be in).
-      bool ok = false;
-      for (uint32_t k = 0; k < kNode2vecTrialsPerCall && !ok; ++k) {
-        if (k) ++s.t;
-        const Rand4 a = philox(s.i, s.j, 2 * s.t + 1, J.job, J.k0, J.k1);
-        if ((unsigned long long)a.y < s.region) {
-          x = (uint32_t)s.prev;
-          ok = true;
-        } else {
-          x = sample_at(W, R, philox(s.i, s.j, 2 * s.t, J.job, J.k0, J.k1));
-          ++s.trials;
-          const unsigned long long io_min = J.thr_in < J.thr_out ? J.thr_in : J.thr_out;
-          if ((int32_t)x == s.prev) {
-            ok = a.x < J.thr_ret;
-          } else if (a.x < io_min) {
-            ok = true;
-          } else {
-            ok = a.x < (hash_has(W.hash + s.phoff, s.phmask, x) ? J.thr_in : J.thr_out);
-            ++s.probes;
-          }
-          ok = ok || s.t + 1 == kMaxNode2vecTrials;
-        }
-      }
-      if (!ok) {
-        ++s.t;
-        return true;  // the step continues on the next call
-      }
-      s.t = 0;
-    } else {
-      x = sample_at(W, R, philox(s.i, s.j, 0, J.job, J.k0, J.k1));
-    }
-    stage_put(o, J.out, obuf, g0 + s.pos, (int32_t)x);
-    ++moves;
-    if (APP == APP_NODE2VEC) {
-      s.prev = (int32_t)s.cur;
-      s.phoff = R.hoff;
-      s.phmask = R.hmask;
-    }
-    s.cur = x;
-    if (APP == APP_PPR && (unsigned long long)philox(s.i, s.j, 1, J.job, J.k0, J.k1).x < J.thr_stop) done = true;
-    ++s.j;
-    if ((s.j >= L && !tail) || (tail && s.j >= kMaxPprSteps)) done = true;
-  }
-  if (done) stage_pad(o, J.out, obuf, g0 + s.pos + 1, g0 + L);
-  return !done;
+  Rand4 r = philox(s.i, s.j, 0, J.job, J.k0, J.k1);
+  uint32_t ax = 0;
+  if (APP == APP_PPR) ax = philox(s.i, s.j, 1, J.job, J.k0, J.k1).x;
+  asm volatile("" : "+r"(r.x), "+r"(r.y), "+r"(r.z), "+r"(r.w), "+r"(ax));  // drawn before R is looked at
+  Proposal p{-1, true, false, 0, 0};
+  if (APP == APP_PPR) p.stop = (unsigned long long)ax < J.thr_stop;
+  if (R.m) p.x = (int32_t)sample_at(W, R.aoff, R.m, r);
+  return p;
 }
 
-__device__ __forceinline__ bool begin_any(const WalkView& W, const WalkJobDev& J, uint32_t i, LaneWalk& s,
-                                          RowStage& o, int32_t (*obuf)[8], uint32_t& mv) {
-  switch (J.app) {
-    case APP_DEEPWALK: return walk_begin<APP_DEEPWALK>(W, J, i, s, o, obuf, mv);
-    case APP_NODE2VEC: return walk_begin<APP_NODE2VEC>(W, J, i, s, o, obuf, mv);
-    case APP_PPR: return walk_begin<APP_PPR>(W, J, i, s, o, obuf, mv);
-    default: return walk_begin<APP_SAMPLING>(W, J, i, s, o, obuf, mv);
+// node2vec steps: the warp draws trials together. A step proposes vertices
+// until one is accepted; each proposal is a chain of three dependent reads,
+// and how many a step takes differs from lane to lane. Which trials a step
+// needs is nearly known before any read: few proposals are the previous
+// vertex or its neighbours, so the first trial whose acceptance draw accepts
+// any other vertex is mostly the one taken. The warp therefore lists every
+// lane's trials up to that one, hands them out one per lane, 32 at a time,
+// and each walk takes its lowest accepted trial (or goes on with the next
+// ones): the same walk as one trial after another, with full warps of reads
+// in flight and, at the end of a launch, the few walks left spread over the
+// warp. First-order walks of a mixed table list their one draw, so that all
+// lanes of a mixed warp read together. Bound: random DRAM reads (the
+// adjacency lookups above all). R-MAT 20, 1 M walks x 40, p = 0.5, q = 2:
+// 2550 us with up to three trials in turn per lane, 1979 us; 16 mixed jobs
+// (1.1 M walks, up to 173 steps, q up to 4): 3960 and 1845 us.
+constexpr uint32_t kTrialItems = 128;  // trials a warp lists per step
+constexpr uint32_t kTrialMax = 16;     // trials a lane lists per step at most
+
+struct TrialScratch {
+  uint32_t ax[kTrialItems];    // acceptance draws, [active lane][trial]
+  uint16_t item[kTrialItems];  // lane | trial << 8 | node2vec trial << 15
+};
+
+// One step of every active lane's walk; `jobs` is the job table (jid indexes
+// it) or the one job.
+template <int APP>
+__device__ __forceinline__ Proposal warp_propose(const WalkView& W, const WalkJobDev* __restrict__ jobs, uint32_t jid,
+                                                 LaneWalk& s, bool active, TrialScratch& sc) {
+  const uint32_t lane = threadIdx.x & 31;
+  const WalkJobDev& J = jobs[jid];
+  const int app = APP >= 0 ? APP : J.app;
+  VertexRec R{0, 0, 0, 0};
+  if (active) R = load_vrec(W, s.cur);
+  const bool n2v = active && app == APP_NODE2VEC && s.prev >= 0;
+  // Trials listed per lane: all lanes' lists fit the scratch.
+  const uint32_t am = __ballot_sync(kFull, active), na = __popc(am);
+  const uint32_t cap = min(kTrialMax, na > 16 ? kTrialItems / 32 : kTrialItems >> (32 - __clz((na - 1) | 1)));
+  const uint32_t mine = __popc(am & lanemask_lt()) * cap;  // this lane's acceptance draws in the scratch
+  Proposal p{-1, true, false, 0, 0};
+  uint32_t n = active ? 1u : 0u;  // trials listed
+  if (n2v || (active && app == APP_PPR)) {
+    n = 0;
+    bool more;
+    do {
+      const uint32_t ax = philox(s.i, s.j, 2 * (s.t + n) + 1, J.job, J.k0, J.k1).x;
+      more = false;
+      if (APP < 0 && app == APP_PPR) {
+        p.stop = (unsigned long long)ax < J.thr_stop;
+      } else {
+        sc.ax[mine + n] = ax;
+        more = ax >= J.thr_out && n + 1 < cap && s.t + n + 1 < kMaxNode2vecTrials;
+      }
+      ++n;
+    } while (more);
   }
+  p.hoff = R.hoff, p.hmask = R.hmask;
+  if (!R.m) n = 0;
+  // A new step's return-region lookup (below) starts here, beside the trials.
+  const bool ret = n2v && R.m && s.t == 0 && J.ret_excess > 0.0;
+  HashPeek rp;
+  if (ret) hash_peek(rp, W.hash + R.hoff, R.hmask, (uint32_t)s.prev);
+  const uint32_t incl = warp_incl_scan(n, lane), off = incl - n;
+  const uint32_t total = __shfl_sync(kFull, incl, 31);
+  for (uint32_t k = 0; k < n; ++k) sc.item[off + k] = (uint16_t)(lane | k << 8 | (n2v ? 1u << 15 : 0u));
+  __syncwarp();
+  constexpr uint32_t kNone = 0xffffffffu;
+  uint32_t won = kNone, probed = 0;  // the accepted trial; this lane's trials that looked up the adjacency index
+  for (uint32_t base = 0; base < total; base += 32) {
+    const bool valid = base + lane < total;
+    const uint32_t it = valid ? sc.item[base + lane] : 0u;
+    const int src = it & 31;
+    const uint32_t vi = __shfl_sync(kFull, s.i, src), vj = __shfl_sync(kFull, s.j, src);
+    const uint32_t vt = __shfl_sync(kFull, s.t, src) + ((it >> 8) & 0x7f);
+    const uint32_t vaoff = __shfl_sync(kFull, R.aoff, src), vm = __shfl_sync(kFull, R.m, src);
+    const int32_t vprev = __shfl_sync(kFull, s.prev, src);
+    const uint32_t vphoff = __shfl_sync(kFull, s.phoff, src), vphmask = __shfl_sync(kFull, s.phmask, src);
+    const WalkJobDev& V = jobs[__shfl_sync(kFull, jid, src)];
+    int32_t x = -1;
+    bool ok = valid, probe = false;
+    if (valid) x = (int32_t)sample_at(W, vaoff, vm, philox(vi, vj, 2 * vt, V.job, V.k0, V.k1));
+    if (it >> 15) {
+      // Accepted with probability weight(class(x)) / envelope; the adjacency
+      // index is read only where the class decides.
+      const unsigned long long ax = sc.ax[__popc(am & ((1u << src) - 1u)) * cap + ((it >> 8) & 0x7f)];
+      if (x == vprev) {
+        ok = ax < V.thr_ret;
+      } else if (ax >= (V.thr_in < V.thr_out ? V.thr_in : V.thr_out)) {
+        probe = true;
+        ok = ax < (hash_has(W.hash + vphoff, vphmask, (uint32_t)x) ? V.thr_in : V.thr_out);
+      }
+      ok = ok || vt + 1 == kMaxNode2vecTrials;
+    }
+    const uint32_t oks = __ballot_sync(kFull, ok), probes = __ballot_sync(kFull, probe);
+    const uint32_t lo = max(off, base), hi = min(off + n, base + 32);
+    int from = 0;
+    bool take = false;
+    if (lo < hi && won == kNone) {  // this lane's trials among the 32
+      const uint32_t here = kFull >> (32 - (hi - lo)), first = lo - base;
+      const uint32_t acc = (oks >> first) & here;
+      probed |= ((probes >> first) & here) << (lo - off);
+      if (acc) {
+        from = (int)(first + __ffs(acc) - 1);
+        won = base + from - off;
+        take = true;
+      }
+    }
+    x = __shfl_sync(kFull, x, from);
+    if (take) p.x = x;
+  }
+  if (n2v && R.m) {
+    // Return region: when 1/p exceeds the envelope max(1, 1/q), the excess
+    // mass (ret_excess x w(cur -> prev)) returns to prev directly, with
+    // probability D / (T + D) per trial (word y of the acceptance block): the
+    // first trial in the region ends the step unless an earlier one did.
+    if (s.t == 0) {
+      s.region = 0;
+      if (ret) {
+        const int e = hash_settle(rp, W.hash + R.hoff, R.hmask, (uint32_t)s.prev);
+        ++s.probes;
+        if (e >= 0 && __ldg(&W.hash[R.hoff + e].cnt) > 0) {
+          const unsigned long long wp = __ldg(&W.hash[R.hoff + e].wsum);
+          const double T = (double)__ldg(&W.alias[R.aoff].T);
+          const double D = __dmul_rn(J.ret_excess, (double)wp);
+          s.region = prob_threshold_dev(__ddiv_rn(D, __dadd_rn(T, D)));
+        }
+      }
+    }
+    uint32_t drawn = won == kNone ? n : won + 1;  // trials up to the accepted one
+    p.ok = won != kNone;
+    if (s.region) {
+      const uint32_t upto = drawn;
+      for (uint32_t k = 0; k < upto; ++k)
+        if ((unsigned long long)philox(s.i, s.j, 2 * (s.t + k) + 1, J.job, J.k0, J.k1).y < s.region) {
+          p.x = s.prev;
+          p.ok = true;
+          drawn = k;
+          break;
+        }
+    }
+    s.trials += drawn;
+    s.probes += __popc(probed & ((1u << drawn) - 1u));
+    if (!p.ok) s.t += n;
+  }
+  __syncwarp();  // the scratch is free for the next step
+  return p;
 }
-__device__ __forceinline__ bool advance_any(const WalkView& W, const WalkJobDev& J, LaneWalk& s, RowStage& o,
-                                            int32_t (*obuf)[8], uint32_t& mv) {
-  switch (J.app) {
-    case APP_DEEPWALK: return walk_advance<APP_DEEPWALK>(W, J, s, o, obuf, mv);
-    case APP_NODE2VEC: return walk_advance<APP_NODE2VEC>(W, J, s, o, obuf, mv);
-    default: return walk_advance<APP_PPR>(W, J, s, o, obuf, mv);
+
+// Takes the proposal as the walk's next move. Returns false when the walk has
+// ended; `out` is set when the row's open line must be written (RowStage::
+// flush up to row position `pos`).
+template <int APP, int LINE>
+__device__ __forceinline__ bool walk_commit(const WalkJobDev& J, LaneWalk& s, const Proposal& p, int32_t* buf,
+                                            uint32_t& moves, bool& out, uint32_t& pos) {
+  const int app = APP >= 0 ? APP : J.app;
+  const bool tail = app == APP_PPR && (J.flags & kWalkPprTail);
+  const uint32_t L = J.L;
+  pos = s.j < L ? s.j : L - 1;
+  const uint32_t at = RowStage<LINE>::slot(s.row + pos);
+  bool done = p.x < 0;
+  buf[at] = p.x;
+  if (!done) {
+    ++moves;
+    if (app == APP_NODE2VEC) {
+      s.prev = (int32_t)s.cur;
+      s.phoff = p.hoff;
+      s.phmask = p.hmask;
+      s.t = 0;
+    }
+    s.cur = (uint32_t)p.x;
+    ++s.j;
+    done = p.stop || (s.j >= L && !tail) || (tail && s.j >= kMaxPprSteps);
   }
+  // A tail walk rewrites its last position until it stops.
+  out = done || (at == LINE - 1 && !(tail && pos == L - 1));
+  return !done;
 }
 
 // One atomic per warp: adds the warp's produced steps to the running count.
