@@ -137,27 +137,59 @@ __host__ __device__ inline uint32_t plan_blocks(uint32_t ks) { return (ks + kPla
 // block (excl[s], s < ks) and each block's sums, column-major per arena
 // (bsum[a * nb + block]); segments past the last one need nothing. A
 // segment's offset in arena a is then the prefix of bsum over blocks (which
-// k_totals writes in place) plus excl[s].
+// k_totals writes in place) plus excl[s]. Segments for a whole block of the
+// apply kernel carry kBigFlag there and are listed in big[0..ctl[1]).
 __global__ void __launch_bounds__(kPlanThreads) k_plan(StoreView S, const uint32_t* skey, const uint32_t* sw,
                                                        const uint32_t* seg, const uint32_t* nseg,
-                                                       unsigned long long k, uint32_t ks, const uint32_t* ctl,
-                                                       ArenaNeed* excl, unsigned long long* bsum) {
+                                                       unsigned long long k, uint32_t ks, uint32_t* ctl,
+                                                       ArenaNeed* excl, unsigned long long* bsum, uint32_t* big) {
   pdl_wait();
   pdl_trigger();
   __shared__ unsigned long long nd_s[kPlanSegs][kArenas];
+  __shared__ uint32_t lcnt[kBits], lpc, lb[kPlanSegs], le[kPlanSegs], bigs;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const uint32_t s = blockIdx.x * kPlanSegs + w;
   const uint32_t nS = *nseg;
   unsigned long long nd[kArenas] = {0, 0, 0, 0, 0};
+  uint32_t b = 0, e = 0, u = 0xffffffffu;
   if (*ctl == 0 && s < nS) {
-    uint32_t b, e;
     seg_bounds(seg, nS, s, k, &b, &e);
-    const uint32_t u = skey[b];
-    if (u < S.n) plan_append(S, u, sw + b, e - b, nd);
+    u = skey[b];
+  }
+  const bool seg_ok = u < S.n, lng = seg_ok && e - b > kBigLen;
+  bool by_block = false;
+  if (threadIdx.x == 0) bigs = 0;
+  if (seg_ok && !lng) {
+    uint32_t add, pc;
+    count_bits(lane, sw + b, e - b, &add, &pc);
+    by_block = plan_append(S, u, e - b, add, pc, nd);
+  }
+  // Long segments: the whole block counts each one's bits.
+  if (lane == 0) lb[w] = b, le[w] = lng ? e : b;
+  if (__syncthreads_or(lng)) {
+    for (int v = 0; v < kPlanSegs; ++v) {
+      const uint32_t vb = lb[v], ve = le[v];
+      if (vb == ve) continue;
+      if (w == 0) lcnt[lane] = 0, lpc = 0;
+      __syncthreads();
+      const uint32_t per = ((ve - vb + 31) / 32 + kPlanSegs - 1) / kPlanSegs * 32;
+      const uint32_t from = min(ve, vb + w * per), to = min(ve, from + per);
+      uint32_t add, pc;
+      count_bits(lane, sw + from, to - from, &add, &pc);
+      if (add) atomicAdd(&lcnt[lane], add);
+      if (lane == 0 && pc) atomicAdd(&lpc, pc);
+      __syncthreads();
+      if (w == v) by_block = plan_append(S, u, e - b, lcnt[lane], lpc, nd);
+      __syncthreads();
+    }
   }
   if (lane == 0) {
 #pragma unroll
     for (int a = 0; a < kArenas; ++a) nd_s[w][a] = nd[a];
+    if (by_block) {
+      big[atomicAdd(ctl + 1, 1u)] = s;
+      atomicOr(&bigs, 1u << w);
+    }
   }
   __syncthreads();
   if (w == 0) {  // lane v: the block's segment v
@@ -171,7 +203,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_plan(StoreView S, const uint32
         const unsigned long long z = __shfl_up_sync(kFull, yi, o);
         if (lane >= o) yi += z;
       }
-      if (sv < ks) excl[sv].v[a] = yi - y;
+      if (sv < ks) excl[sv].v[a] = (yi - y) | (a == A_EDGE && ((bigs >> lane) & 1u) ? kBigFlag : 0ull);
       if (lane == 31) bsum[(size_t)a * nb + blockIdx.x] = yi;
     }
   }
@@ -318,24 +350,40 @@ __global__ void __launch_bounds__(kBlock, 4) k_apply_insert(StoreView S, const u
                                                          unsigned long long k, uint32_t ks, const uint32_t* ctl,
                                                          const ArenaNeed* excl, const unsigned long long* boff,
                                                          const unsigned long long* base, HostReserve hr,
-                                                         uint32_t* out_slots) {
+                                                         const uint32_t* big, uint32_t* out_slots) {
+  static_assert(kBlock / 32 == kAppendWarps, "a block appends a listed segment");
   pdl_wait();
   pdl_trigger();
   __shared__ AliasScratch asc[kBlock / 32];
+  __shared__ BlockAppend ba;
   if (*ctl) return;
   if (!base && blockIdx.x == 0) {
 #pragma unroll
     for (int a = 0; a < kArenas; ++a)
       if (threadIdx.x == a) S.top[a] = hr.top[a];  // constant indices keep hr in parameter space
   }
-  const uint32_t warps = gridDim.x * blockDim.x / 32;
-  const uint32_t nS = *nseg, nb = plan_blocks(ks);
-  for (uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) / 32; s < nS; s += warps) {
+  const uint32_t nS = *nseg, nb = plan_blocks(ks), nbig = ctl[1];
+  for (uint32_t q = blockIdx.x; q < nbig; q += gridDim.x) {
+    const uint32_t s = big[q];
+    uint32_t b, e;
+    seg_bounds(seg, nS, s, k, &b, &e);
+    unsigned long long res[kArenas];
+    for (int a = 0; a < kArenas; ++a)
+      res[a] = (base ? base[a] : hr.base[a]) + boff[(size_t)a * nb + s / kPlanSegs] + (excl[s].v[a] & ~kBigFlag);
+    apply_append_block(S, skey[b], sv + b, sw + b, sorig + b, e - b, out_slots, res, &asc[threadIdx.x / 32], ba);
+  }
+  // The other segments, one warp each; blocks that had a listed one leave them
+  // to the rest while those are the most.
+  const uint32_t skip = nbig < gridDim.x / 2 ? nbig : 0u;
+  if (blockIdx.x < skip) return;
+  const uint32_t warps = (gridDim.x - skip) * (blockDim.x / 32);
+  for (uint32_t s = ((blockIdx.x - skip) * blockDim.x + threadIdx.x) / 32; s < nS; s += warps) {
     uint32_t b, e;
     seg_bounds(seg, nS, s, k, &b, &e);
     const uint32_t u = skey[b];
     if (u >= S.n) continue;
     const ArenaNeed off = excl[s];
+    if (off.v[A_EDGE] & kBigFlag) continue;
     unsigned long long res[kArenas];
 #pragma unroll
     for (int a = 0; a < kArenas; ++a)
@@ -825,7 +873,7 @@ Engine::~Engine() {
   drop_graph();
   prog_jobs_.release(), prog_prefix_.release(), prog_queue_.release();
   DevBuf* bufs[] = {&vrec_, &meta_, &gdesc_, &gs_, &in_a_, &in_b_, &in_c_, &key_s_, &perm_, &iota_, &sa_,
-                    &sb_, &head_, &seg_, &nseg_, &need_, &scan_, &base_, &ctl_, &slots_, &cub_tmp_, &jobs_,
+                    &sb_, &head_, &seg_, &nseg_, &need_, &scan_, &big_, &base_, &ctl_, &slots_, &cub_tmp_, &jobs_,
                     &prefix_, &queue_, &wstart_, &wout_[0], &wout_[1], &pair_key_, &pair_key_s_, &pair_slot_,
                     &fw_in_, &fw_fixed_, &check_buf_, &check_big_};
   for (DevBuf* b : bufs) b->release();
@@ -927,6 +975,7 @@ void Engine::ensure_batch_scratch(uint64_t k) {
   base_.ensure(kArenas * 8 * 2, "scratch");
   need_.ensure((size_t)plan_blocks((uint32_t)ks) * sizeof(ArenaNeed), "scratch");  // plan-block sums
   scan_.ensure((size_t)ks * sizeof(ArenaNeed), "scratch");                                   // in-block offsets
+  big_.ensure((size_t)ks * 4, "scratch");
   if (iota_n_ < kk) {
     iota_.ensure(kk * 4, "scratch");
     k_iota<<<grid_for(kk, kBlock), kBlock, 0, stream_>>>(iota_.as<uint32_t>(), kk);
@@ -1118,7 +1167,8 @@ unsigned long long* Engine::plan_needs(const StoreView& S, uint64_t k, uint32_t 
                                        volatile unsigned long long* publish, int reserve) {
   const uint32_t nb = plan_blocks(ks);
   launch_pdl(k_plan, nb, kPlanThreads, stream_, S, key_s_.as<uint32_t>(), sb_.as<uint32_t>(), seg_.as<uint32_t>(),
-             nseg_.as<uint32_t>(), k, ks, ctl_.as<uint32_t>(), scan_.as<ArenaNeed>(), need_.as<unsigned long long>());
+             nseg_.as<uint32_t>(), k, ks, ctl_.as<uint32_t>(), scan_.as<ArenaNeed>(), need_.as<unsigned long long>(),
+             big_.as<uint32_t>());
   cuda_check(cudaGetLastError(), "plan");
   ++launches_;
   unsigned long long* d_tot = base_.as<unsigned long long>() + kArenas;
@@ -1165,7 +1215,7 @@ void Engine::run_insert(uint64_t k, uint32_t* dev_out_slots, bool load_mode, uin
     launch_pdl(k_apply_insert, grid_for((unsigned long long)ks * 32, kBlock, tuning_.apply_blocks_per_sm), kBlock,
                stream_, S, key_s_.as<uint32_t>(), sa_.as<uint32_t>(), sb_.as<uint32_t>(), perm_.as<uint32_t>(),
                seg_.as<uint32_t>(), nseg_.as<uint32_t>(), k, ks, ctl_.as<uint32_t>(), scan_.as<ArenaNeed>(),
-               need_.as<unsigned long long>(), dev_base, hr, dev_out_slots);
+               need_.as<unsigned long long>(), dev_base, hr, big_.as<uint32_t>(), dev_out_slots);
     cuda_check(cudaGetLastError(), "apply insert");
     ++launches_;
   };
@@ -1255,7 +1305,7 @@ void Engine::load(const uint32_t* src, const uint32_t* dst, const uint32_t* w, u
   loaded_ = true;
   // Release load-sized scratch; update batches re-grow what they need.
   DevBuf* big[] = {&in_a_, &in_b_, &in_c_, &key_s_, &perm_, &sa_, &sb_, &head_, &seg_, &slots_, &need_,
-                   &scan_, &iota_, &cub_tmp_};
+                   &scan_, &big_, &iota_, &cub_tmp_};
   cuda_check(cudaStreamSynchronize(stream_), "load");
   for (DevBuf* b : big) b->release();
   iota_n_ = 0;
@@ -1669,7 +1719,7 @@ void Engine::enqueue_insert(const uint32_t* a, const uint32_t* b, const uint32_t
   launch_pdl(k_apply_insert, grid_for((unsigned long long)ks * 32, kBlock, tuning_.apply_blocks_per_sm), kBlock,
              stream_, S, key_s_.as<uint32_t>(), sa_.as<uint32_t>(), sb_.as<uint32_t>(), perm_.as<uint32_t>(),
              seg_.as<uint32_t>(), nseg_.as<uint32_t>(), k, ks, ctl_.as<uint32_t>(), scan_.as<ArenaNeed>(),
-             need_.as<unsigned long long>(), base_.as<unsigned long long>(), HostReserve{}, out_slots);
+             need_.as<unsigned long long>(), base_.as<unsigned long long>(), HostReserve{}, big_.as<uint32_t>(), out_slots);
   cuda_check(cudaGetLastError(), "apply insert");
   ++launches_;
 }
@@ -2026,7 +2076,7 @@ void Engine::stats(bingo_stats* out) {
     out->arena_used += h_top_[a] * kUnitBytes[a] + (a == A_MEMBER ? h_top_[a] * 4 : 0);
   }
   const DevBuf* sc[] = {&in_a_, &in_b_, &in_c_, &key_s_, &perm_, &iota_, &sa_, &sb_, &head_, &seg_, &nseg_,
-                        &need_, &scan_, &base_, &ctl_, &slots_, &cub_tmp_, &jobs_, &prefix_, &queue_, &wstart_,
+                        &need_, &scan_, &big_, &base_, &ctl_, &slots_, &cub_tmp_, &jobs_, &prefix_, &queue_, &wstart_,
                         &wout_[0], &wout_[1], &pair_key_, &pair_key_s_, &pair_slot_, &fw_in_, &fw_fixed_,
                         &prog_jobs_, &prog_prefix_, &prog_queue_};
   for (const DevBuf* b : sc) out->scratch_bytes += b->bytes;

@@ -146,7 +146,7 @@ class Engine {
   unsigned long long launches_ = 0;        // hand-written kernels launched since create
 
   // per-batch scratch
-  DevBuf in_a_, in_b_, in_c_, key_s_, perm_, iota_, sa_, sb_, head_, seg_, nseg_, need_, scan_, base_, ctl_,
+  DevBuf in_a_, in_b_, in_c_, key_s_, perm_, iota_, sa_, sb_, head_, seg_, nseg_, need_, scan_, big_, base_, ctl_,
       slots_, cub_tmp_;
   DevBuf pair_key_, pair_key_s_, pair_slot_;  // delete-by-pair translation
   DevBuf fw_in_, fw_fixed_;                   // float weights: staged input, 16.16 fixed point

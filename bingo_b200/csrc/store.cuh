@@ -261,6 +261,62 @@ __device__ __forceinline__ void warp_copy_u32(uint32_t* dst, const uint32_t* src
   warp_copy_v4(reinterpret_cast<uint4*>(dst), reinterpret_cast<const uint4*>(src), (n + 3) / 4, lane);
 }
 
+// Appends edges [from, to) of a segment in batch order (one warp): M with the
+// vertex's arrays and its slot count before the segment; G.cnt and bpbase are
+// the positions this range starts at and end past it. `single` becomes the
+// first member of a group that was empty.
+__device__ __forceinline__ void append_range(const StoreView& S, const VertexMeta& M, GroupDesc& G, uint32_t& bpbase,
+                                             uint32_t& single, const uint32_t* seg_v, const uint32_t* seg_w,
+                                             const uint32_t* seg_orig, uint32_t from, uint32_t to,
+                                             uint32_t* out_slots) {
+  const int lane = threadIdx.x & 31;
+  for (uint32_t c = from; c < to; c += 32) {
+    const uint32_t i = c + lane;
+    const bool valid = i < to;
+    const uint32_t v = valid ? seg_v[i] : 0u, w = valid ? seg_w[i] : 0u;
+    const uint32_t pc = __popc(w);
+    const uint32_t incl = warp_incl_scan(pc, lane);
+    const uint32_t ebp = bpbase + incl - pc;
+    bpbase += __shfl_sync(kFull, incl, 31);
+    const uint32_t slot = M.ecnt + i;
+    if (valid) {
+      S.edges[M.eoff + slot] = EdgeRec{v, w, ebp, 0u};
+      if (out_slots) out_slots[seg_orig[i]] = slot;
+    }
+    uint32_t present = __reduce_or_sync(kFull, w);
+    while (present) {
+      const int k = __ffs(present) - 1;
+      present &= present - 1;
+      const bool has = (w >> k) & 1u;
+      const uint32_t b = __ballot_sync(kFull, has);
+      const uint32_t kcnt = __shfl_sync(kFull, G.cnt, k), kbase = __shfl_sync(kFull, group_base(G), k);
+      if (has) {
+        const uint32_t pos = kcnt + __popc(b & lanemask_lt()), bi = ebp + __popc(w & ((1u << k) - 1u));
+        const size_t e = (size_t)kbase * 4 + pos;
+        S.gv[e] = v;
+        S.gs[e] = bi;
+        S.bp[M.bpoff + bi] = pos;
+      }
+      const uint32_t first_v = __shfl_sync(kFull, v, __ffs(b) - 1);  // b != 0: bit k is present
+      if (lane == k) {
+        if (kcnt == 0) single = first_v;
+        G.cnt += __popc(b);
+      }
+    }
+  }
+}
+
+// Segments a whole block appends (apply_append_block) instead of one warp:
+// long ones, and those whose vertex moves a large store. One warp appends 32
+// edges or copies 1 KB per round trip, so a hub alone set the kernel's time:
+// R-MAT 20's largest vertex kept its load apply running for 6.9 ms.
+// (Lines: a warp takes about 3 us per 32 edges and a block 10 us to share a
+// segment out. Measured, R-MAT 20: load apply 6.9 ms to 2.9; 50K-edge insert
+// batches whose vertices follow the degree, 130 us to 79.)
+constexpr uint32_t kBigLen = 256;          // edges
+constexpr uint32_t kBigCopy = 1024;        // 16-byte units copied by relocations
+constexpr unsigned long long kBigFlag = 1ull << 63;  // marks such a segment in its A_EDGE offset
+
 // ---------------------------------------------------------------------------
 // Apply a growth plan (relocations drawn from per-arena bases reserved for
 // this segment), append the segment's edges in order, refresh the adjacency
@@ -344,40 +400,8 @@ static __device__ void apply_append(const StoreView& S, uint32_t u, const uint32
       ++G.cnt;
     }
     bpbase += __popc(w);
-  }
-  for (uint32_t c = 0; len > 1 && c < len; c += 32) {
-    const uint32_t i = c + lane;
-    const bool valid = i < len;
-    const uint32_t v = valid ? seg_v[i] : 0u, w = valid ? seg_w[i] : 0u;
-    const uint32_t pc = __popc(w);
-    const uint32_t incl = warp_incl_scan(pc, lane);
-    const uint32_t ebp = bpbase + incl - pc;
-    bpbase += __shfl_sync(kFull, incl, 31);
-    const uint32_t slot = M.ecnt + i;
-    if (valid) {
-      S.edges[M.eoff + slot] = EdgeRec{v, w, ebp, 0u};
-      if (out_slots) out_slots[seg_orig[i]] = slot;
-    }
-    uint32_t present = __reduce_or_sync(kFull, w);
-    while (present) {
-      const int k = __ffs(present) - 1;
-      present &= present - 1;
-      const bool has = (w >> k) & 1u;
-      const uint32_t b = __ballot_sync(kFull, has);
-      const uint32_t kcnt = __shfl_sync(kFull, G.cnt, k), kbase = __shfl_sync(kFull, group_base(G), k);
-      if (has) {
-        const uint32_t pos = kcnt + __popc(b & lanemask_lt()), bi = ebp + __popc(w & ((1u << k) - 1u));
-        const size_t e = (size_t)kbase * 4 + pos;
-        S.gv[e] = v;
-        S.gs[e] = bi;
-        S.bp[M.bpoff + bi] = pos;
-      }
-      const uint32_t first_v = __shfl_sync(kFull, v, __ffs(b) - 1);  // b != 0: bit k is present
-      if (lane == k) {
-        if (kcnt == 0) single = first_v;
-        G.cnt += __popc(b);
-      }
-    }
+  } else {
+    append_range(S, M, G, bpbase, single, seg_v, seg_w, seg_orig, 0, len, out_slots);
   }
   M.ecnt += len;
   M.bpcnt = bpbase;
@@ -417,21 +441,162 @@ static __device__ void apply_append(const StoreView& S, uint32_t u, const uint32
   }
 }
 
+// Block copy of n 16-byte units between non-overlapping ranges, four loads per
+// lane in flight.
+__device__ __forceinline__ void block_copy_v4(uint4* __restrict__ dst, const uint4* __restrict__ src, uint32_t n) {
+  const uint32_t T = blockDim.x;
+  uint32_t i = threadIdx.x;
+  for (; i + 3 * T < n; i += 4 * T) {
+    const uint4 a = src[i], b = src[i + T], c = src[i + 2 * T], d = src[i + 3 * T];
+    dst[i] = a, dst[i + T] = b, dst[i + 2 * T] = c, dst[i + 3 * T] = d;
+  }
+  for (; i < n; i += T) dst[i] = src[i];
+}
+__device__ __forceinline__ void block_copy_u32(uint32_t* dst, const uint32_t* src, uint32_t n) {
+  block_copy_v4(reinterpret_cast<uint4*>(dst), reinterpret_cast<const uint4*>(src), (n + 3) / 4);
+}
+
+constexpr int kAppendWarps = 8;  // warps of a block that appends one segment
+struct BlockAppend {
+  uint32_t cnt[kAppendWarps][kBits];  // bit counts per warp's range, then its first positions
+  uint32_t pc[kAppendWarps];          // popcount sums per warp's range
+  uint32_t single[kBits];             // first member of a group that was empty
+  uint32_t claimed;                   // adjacency keys added
+};
+
+// apply_append by a block of kAppendWarps warps: each warp takes a contiguous
+// range of the segment, counts its bits, and appends at the positions that
+// the ranges before it leave; the block shares the copies of moved arrays and
+// the adjacency updates. The store is the one apply_append leaves.
+static __device__ __noinline__ void apply_append_block(const StoreView& S, uint32_t u, const uint32_t* seg_v,
+                                                       const uint32_t* seg_w, const uint32_t* seg_orig, uint32_t len,
+                                                       uint32_t* out_slots, const unsigned long long res[kArenas],
+                                                       AliasScratch* sc, BlockAppend& B) {
+  const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+  VertexMeta M = S.meta[u];
+  GroupDesc G = S.gdesc[(size_t)u * kBits + lane];
+  VertexRec R = S.vrec[u];
+  const uint32_t cap0 = group_cap(G), cnt0 = G.cnt;
+  // Ranges of whole 32-edge chunks.
+  const uint32_t per = ((len + 31) / 32 + kAppendWarps - 1) / kAppendWarps * 32;
+  const uint32_t from = min(len, wi * per), to = min(len, from + per);
+  uint32_t add, pc;
+  count_bits(lane, seg_w + from, to - from, &add, &pc);
+  B.cnt[wi][lane] = add;
+  if (lane == 0) B.pc[wi] = pc;
+  if (wi == 0) {
+    B.single[lane] = G.cnt == 1 ? S.gv[(size_t)group_base(G) * 4] : 0u;
+    if (lane == 0) B.claimed = 0;
+  }
+  __syncthreads();
+  uint32_t add_lane = 0, pc_total = 0, before = 0, pc_before = 0;
+#pragma unroll
+  for (int v = 0; v < kAppendWarps; ++v) {
+    if (v == wi) before = add_lane, pc_before = pc_total;
+    add_lane += B.cnt[v][lane];
+    pc_total += B.pc[v];
+  }
+  const GrowPlan P = plan_growth(lane, M, G, len, add_lane, pc_total, S.node2vec);
+  // --- relocations (old contents keep their order) ---
+  if (P.new_ecap) {
+    block_copy_v4(reinterpret_cast<uint4*>(S.edges + res[A_EDGE]), reinterpret_cast<const uint4*>(S.edges + M.eoff),
+                  M.ecnt);
+    M.eoff = res[A_EDGE];
+    M.ecap = P.new_ecap;
+  }
+  if (P.new_bpcap) {
+    block_copy_u32(S.bp + res[A_BP], S.bp + M.bpoff, M.bpcnt);
+    M.bpoff = res[A_BP];
+    M.bpcap = P.new_bpcap;
+  }
+  {
+    const uint32_t old_base = group_base(G);
+    uint32_t copy = __ballot_sync(kFull, P.gcap_lane != 0 && G.cnt != 0);
+    if (P.gcap_lane) {
+      G.base1 = (uint32_t)((res[A_MEMBER] + P.gpre) >> 2) + 1u;
+      G.roomy = 0;
+    }
+    while (copy) {  // the same lists in every warp
+      const int k = __ffs(copy) - 1;
+      copy &= copy - 1;
+      const uint32_t ob = __shfl_sync(kFull, old_base, k), oc = __shfl_sync(kFull, G.cnt, k);
+      const size_t nb = (size_t)__shfl_sync(kFull, group_base(G), k) * 4;
+      block_copy_u32(S.gv + nb, S.gv + (size_t)ob * 4, oc);
+      block_copy_u32(S.gs + nb, S.gs + (size_t)ob * 4, oc);
+    }
+  }
+  if (P.new_acap) {
+    R.aoff = (uint32_t)res[A_ALIAS];
+    M.acap = P.new_acap;
+  }
+  if (P.new_hcap) {
+    HashEntry* tab = S.hash + res[A_HASH];
+    for (uint32_t i = threadIdx.x; i < P.new_hcap; i += blockDim.x) tab[i] = HashEntry{kEmptyKey, 0, 0ull};
+  }
+  __syncthreads();  // copies round up to 16 bytes: they end before the entries past the old ones are written
+
+  // --- append ---
+  G.cnt += before;
+  uint32_t bpbase = M.bpcnt + pc_before, single = 0xffffffffu;
+  append_range(S, M, G, bpbase, single, seg_v, seg_w, seg_orig, from, to, out_slots);
+  if (cnt0 == 0 && before == 0 && add) B.single[lane] = single;  // this range holds the group's first member
+  M.ecnt += len;
+  M.bpcnt += pc_total;
+  M.live += len;
+  __syncthreads();
+
+  // --- adjacency index ---
+  if (S.node2vec) {
+    uint32_t claimed = 0;
+    if (P.new_hcap) {
+      HashEntry* tab = S.hash + res[A_HASH];
+      for (uint32_t i = threadIdx.x; i < M.ecnt; i += blockDim.x) {
+        const EdgeRec e = S.edges[M.eoff + i];
+        if (e.w) hash_add(tab, P.new_hcap - 1, e.v, e.w, &claimed);
+      }
+      R.hoff = (uint32_t)res[A_HASH];
+      R.hmask = P.new_hcap - 1;
+      M.hcap = P.new_hcap;
+    } else {
+      for (uint32_t i = threadIdx.x; i < len; i += blockDim.x)
+        hash_add(S.hash + R.hoff, R.hmask, seg_v[i], seg_w[i], &claimed);
+    }
+    claimed = warp_sum_u32(claimed);
+    if (lane == 0 && claimed) atomicAdd(&B.claimed, claimed);
+    __syncthreads();
+    M.hkeys = (P.new_hcap ? 0u : M.hkeys) + B.claimed;
+  }
+  // --- alias table over the new counts ---
+  if (wi == 0) {
+    G.cnt = cnt0 + add_lane;
+    R.m = warp_build_alias(lane, G.cnt, group_base(G), B.single[lane], S.alias + R.aoff, sc);
+    if (add_lane && !P.gcap_lane) G.roomy = group_roomy(G.cnt, cap0);
+    if (add_lane || P.gcap_lane) S.gdesc[(size_t)u * kBits + lane] = G;
+    if (lane == 0) {
+      S.meta[u] = M;
+      S.vrec[u] = R;
+    }
+  }
+  __syncthreads();  // B is reused by the block's next segment
+}
+
 // Per-arena sizes the append of a segment needs (same decisions as
-// apply_append). Lane 0 returns them.
-__device__ __forceinline__ void plan_append(const StoreView& S, uint32_t u, const uint32_t* seg_w, uint32_t len,
-                                            unsigned long long need[kArenas]) {
+// apply_append), from its counts (count_bits). Returns whether a block
+// appends it. Called by the whole warp.
+__device__ __forceinline__ bool plan_append(const StoreView& S, uint32_t u, uint32_t len, uint32_t add_lane,
+                                            uint32_t pc_total, unsigned long long need[kArenas]) {
   const int lane = threadIdx.x & 31;
   const VertexMeta M = S.meta[u];
   const GroupDesc G = S.gdesc[(size_t)u * kBits + lane];
-  uint32_t add_lane, pc_total;
-  count_bits(lane, seg_w, len, &add_lane, &pc_total);
   const GrowPlan P = plan_growth(lane, M, G, len, add_lane, pc_total, S.node2vec);
   need[A_MEMBER] = P.gsum;
   need[A_EDGE] = P.new_ecap;
   need[A_BP] = P.new_bpcap;
   need[A_ALIAS] = P.new_acap;
   need[A_HASH] = P.new_hcap;
+  const uint32_t moved = __reduce_add_sync(kFull, P.gcap_lane ? G.cnt / 2 : 0u) + (P.new_ecap ? M.ecnt : 0u) +
+                         (P.new_bpcap ? M.bpcnt / 4 : 0u) + (P.new_hcap ? M.ecnt : 0u);
+  return len > kBigLen || moved > kBigCopy;
 }
 
 // Removals of one group a lane resolves per round of loads (apply_delete).
