@@ -184,7 +184,8 @@ struct GrowPlan {
   uint32_t new_ecap;   // 0 = no edge relocation
   uint32_t new_bpcap;  // 0 = no back-pointer relocation
   uint32_t new_acap;   // 0 = alias table fits
-  uint32_t new_hcap;   // 0 = adjacency index fits
+  uint32_t new_hcap;   // 0 = adjacency index fits its table
+  bool rehash;         // the index is rebuilt (into a new table when new_hcap)
   uint32_t gcap_lane;  // this lane's new group capacity, 0 = fits
   uint32_t gsum;       // sum over lanes of gcap_lane
   uint32_t gpre;       // exclusive prefix of gcap_lane over lanes
@@ -206,8 +207,16 @@ __device__ __forceinline__ GrowPlan plan_growth(int lane, const VertexMeta& M, c
   p.gpre = incl - p.gcap_lane;
   const uint32_t m = __popc(__ballot_sync(kFull, cnt != 0));
   p.new_acap = m > M.acap ? pow2_at_least(m, 1) : 0;
+  // An index whose dead keys (of deleted edges) fill its table is rebuilt in
+  // place; only one whose live keys outgrow the table takes a new one. (A
+  // steady stream of inserts and deletes took a new table of the same size
+  // for a part of its vertices in every batch, until the arena had to grow.)
   p.new_hcap = 0;
-  if (node2vec && (M.hkeys + len > M.hcap / 2)) p.new_hcap = pow2_at_least(2 * (M.live + len), kMinHashCap);
+  p.rehash = node2vec && (M.hkeys + len > M.hcap / 2);
+  if (p.rehash) {
+    const uint32_t want = pow2_at_least(2 * (M.live + len), kMinHashCap);
+    if (want > M.hcap) p.new_hcap = want;
+  }
   return p;
 }
 
@@ -411,18 +420,20 @@ static __device__ void apply_append(const StoreView& S, uint32_t u, const uint32
   // --- adjacency index ---
   if (S.node2vec) {
     uint32_t claimed = 0;
-    if (P.new_hcap) {
-      // Rebuild from every live slot into a fresh table.
-      HashEntry* tab = S.hash + res[A_HASH];
-      for (uint32_t i = lane; i < P.new_hcap; i += 32) tab[i] = HashEntry{kEmptyKey, 0, 0ull};
+    if (P.rehash) {
+      // Rebuild from every live slot into a cleared table.
+      if (P.new_hcap) {
+        R.hoff = (uint32_t)res[A_HASH];
+        R.hmask = P.new_hcap - 1;
+        M.hcap = P.new_hcap;
+      }
+      HashEntry* tab = S.hash + R.hoff;
+      for (uint32_t i = lane; i < M.hcap; i += 32) tab[i] = HashEntry{kEmptyKey, 0, 0ull};
       __syncwarp();
       for (uint32_t i = lane; i < M.ecnt; i += 32) {
         const EdgeRec e = S.edges[M.eoff + i];
-        if (e.w) hash_add(tab, P.new_hcap - 1, e.v, e.w, &claimed);
+        if (e.w) hash_add(tab, R.hmask, e.v, e.w, &claimed);
       }
-      R.hoff = (uint32_t)res[A_HASH];
-      R.hmask = P.new_hcap - 1;
-      M.hcap = P.new_hcap;
       M.hkeys = warp_sum_u32(claimed);
     } else {
       for (uint32_t i = lane; i < len; i += 32) hash_add(S.hash + R.hoff, R.hmask, seg_v[i], seg_w[i], &claimed);
@@ -530,8 +541,13 @@ static __device__ __noinline__ void apply_append_block(const StoreView& S, uint3
     M.acap = P.new_acap;
   }
   if (P.new_hcap) {
-    HashEntry* tab = S.hash + res[A_HASH];
-    for (uint32_t i = threadIdx.x; i < P.new_hcap; i += blockDim.x) tab[i] = HashEntry{kEmptyKey, 0, 0ull};
+    R.hoff = (uint32_t)res[A_HASH];
+    R.hmask = P.new_hcap - 1;
+    M.hcap = P.new_hcap;
+  }
+  if (P.rehash) {
+    HashEntry* tab = S.hash + R.hoff;
+    for (uint32_t i = threadIdx.x; i < M.hcap; i += blockDim.x) tab[i] = HashEntry{kEmptyKey, 0, 0ull};
   }
   __syncthreads();  // copies round up to 16 bytes: they end before the entries past the old ones are written
 
@@ -548,15 +564,11 @@ static __device__ __noinline__ void apply_append_block(const StoreView& S, uint3
   // --- adjacency index ---
   if (S.node2vec) {
     uint32_t claimed = 0;
-    if (P.new_hcap) {
-      HashEntry* tab = S.hash + res[A_HASH];
+    if (P.rehash) {
       for (uint32_t i = threadIdx.x; i < M.ecnt; i += blockDim.x) {
         const EdgeRec e = S.edges[M.eoff + i];
-        if (e.w) hash_add(tab, P.new_hcap - 1, e.v, e.w, &claimed);
+        if (e.w) hash_add(S.hash + R.hoff, R.hmask, e.v, e.w, &claimed);
       }
-      R.hoff = (uint32_t)res[A_HASH];
-      R.hmask = P.new_hcap - 1;
-      M.hcap = P.new_hcap;
     } else {
       for (uint32_t i = threadIdx.x; i < len; i += blockDim.x)
         hash_add(S.hash + R.hoff, R.hmask, seg_v[i], seg_w[i], &claimed);
@@ -564,7 +576,7 @@ static __device__ __noinline__ void apply_append_block(const StoreView& S, uint3
     claimed = warp_sum_u32(claimed);
     if (lane == 0 && claimed) atomicAdd(&B.claimed, claimed);
     __syncthreads();
-    M.hkeys = (P.new_hcap ? 0u : M.hkeys) + B.claimed;
+    M.hkeys = (P.rehash ? 0u : M.hkeys) + B.claimed;
   }
   // --- alias table over the new counts ---
   if (wi == 0) {
@@ -595,7 +607,7 @@ __device__ __forceinline__ bool plan_append(const StoreView& S, uint32_t u, uint
   need[A_ALIAS] = P.new_acap;
   need[A_HASH] = P.new_hcap;
   const uint32_t moved = __reduce_add_sync(kFull, P.gcap_lane ? G.cnt / 2 : 0u) + (P.new_ecap ? M.ecnt : 0u) +
-                         (P.new_bpcap ? M.bpcnt / 4 : 0u) + (P.new_hcap ? M.ecnt : 0u);
+                         (P.new_bpcap ? M.bpcnt / 4 : 0u) + (P.rehash ? M.ecnt + M.hcap / 2 : 0u);
   return len > kBigLen || moved > kBigCopy;
 }
 
