@@ -116,7 +116,7 @@ struct StoreView {
   HashEntry* hash;
   unsigned long long* top;  // [kArenas] bump pointers (arena units)
   unsigned long long cap[kArenas];
-  uint32_t* err;            // [0] ErrBit mask, [1] rejected-delete count
+  uint32_t* err;            // error words (set_err)
   uint32_t node2vec;
 };
 
@@ -187,6 +187,12 @@ __host__ __device__ __forceinline__ uint32_t mix32(uint32_t h) {
   return h;
 }
 
-__device__ __forceinline__ void set_err(uint32_t* err, uint32_t bit) { atomicOr(err, bit); }
+// Error words: [0] ErrBit mask, [1] rejected deletes, [2..3] the device address
+// of a flag in mapped host memory, raised with every error, so that a host
+// that has waited for the stream knows without a copy that there is none.
+__device__ __forceinline__ void set_err(uint32_t* err, uint32_t bits) {
+  atomicOr(err, bits);
+  **reinterpret_cast<volatile unsigned long long* const*>(err + 2) = 1ull;
+}
 
 }  // namespace bingo

@@ -98,7 +98,7 @@ __global__ void k_validate(const uint32_t* a, const uint32_t* b, const uint32_t*
   bits = __reduce_or_sync(kFull, bits);
   if (bits && (threadIdx.x & 31) == 0) {
     atomicOr(ctl, bits);
-    atomicOr(err, bits);
+    set_err(err, bits);
   }
 }
 
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(kTotalsThreads) k_totals(StoreView S, unsigned
       } else {
         st = kReserveFull;
         atomicOr(ctl, E_CAPACITY);
-        if (reserve == kReserveSticky) atomicOr(S.err, E_CAPACITY);
+        if (reserve == kReserveSticky) set_err(S.err, E_CAPACITY);
       }
     }
     status = st;
@@ -481,8 +481,8 @@ __global__ void __launch_bounds__(kBlock) k_pair_slots(StoreView S, const unsign
 
 // Persistent walk kernel with per-lane refill. Each warp owns a range of
 // walk items and hands them to idle lanes; when the range runs out it pulls
-// the next `chunk` items from one device counter (reset by the host before
-// launch). MULTI = false: every item is a walk of the single job J0.
+// the next `chunk` items from one device counter (queue[0], zero at launch
+// and zeroed again by the last warp to finish, which queue[1] counts). MULTI = false: every item is a walk of the single job J0.
 // MULTI = true: items index the concatenated jobs of a device job table
 // (prefix = running walk counts) and each lane follows its own job; APP >= 0
 // when every job of the table has that app, APP < 0 for a mixed table.
@@ -592,6 +592,8 @@ __global__ void __launch_bounds__(kBlock, walk_min_blocks(APP, MULTI))
   }
   add_steps(W, moves);
   add_n2v(W, s);
+  // The last warp leaves the work counter zeroed for the next launch.
+  if (lane == 0 && atomicAdd(queue + 1, 1u) + 1 == warps) queue[0] = queue[1] = 0;
 }
 
 __global__ void k_philox(const uint32_t* ctr, unsigned long long count, uint32_t k0, uint32_t k1, uint32_t* out) {
@@ -861,6 +863,10 @@ Engine::Engine(const bingo_config& cfg) : cfg_(cfg) {
   cuda_check(cudaHostAlloc((void**)&h_plan_, 16 * sizeof(unsigned long long), cudaHostAllocMapped),
              "cudaHostAlloc(plan)");
   cuda_check(cudaHostGetDevicePointer((void**)&d_plan_, (void*)h_plan_, 0), "plan mapping");
+  err_flag_ = h_plan_ + 15;
+  *err_flag_ = 0;
+  const unsigned long long* const d_flag = d_plan_ + 15;
+  cuda_check(cudaMemcpy(d_err_ + 2, &d_flag, sizeof d_flag, cudaMemcpyHostToDevice), "error flag");
   cuda_check(cudaEventCreateWithFlags(&slots_ev_, cudaEventDisableTiming), "cudaEventCreate");
   walk_carveouts(cfg.device);
 }
@@ -875,7 +881,7 @@ Engine::~Engine() {
   DevBuf* bufs[] = {&vrec_, &meta_, &gdesc_, &gs_, &in_a_, &in_b_, &in_c_, &key_s_, &perm_, &iota_, &sa_,
                     &sb_, &head_, &seg_, &nseg_, &need_, &scan_, &big_, &base_, &ctl_, &slots_, &cub_tmp_, &jobs_,
                     &prefix_, &queue_, &wstart_, &wout_[0], &wout_[1], &pair_key_, &pair_key_s_, &pair_slot_,
-                    &fw_in_, &fw_fixed_, &check_buf_, &check_big_};
+                    &fw_in_, &fw_fixed_, &check_buf_, &check_big_, &load_slab_};
   for (DevBuf* b : bufs) b->release();
   for (int k = 0; k < 2; ++k) {
     if (walk_ev_[k]) cudaEventDestroy(walk_ev_[k]);
@@ -931,13 +937,22 @@ void Engine::require_loaded() const {
 
 void Engine::set_stream(void* s) { stream_ = s ? (cudaStream_t)s : own_stream_; }
 
+// Forgets the errors raised so far (their stream has been waited for).
+void Engine::clear_err() {
+  cuda_check(cudaMemset(d_err_, 0, 2 * sizeof(uint32_t)), "clear status");
+  *err_flag_ = 0;
+}
+
 int Engine::sync() {
   cuda_check(cudaStreamSynchronize(stream_), "stream synchronize");
   cuda_check(cudaStreamSynchronize(xstream_), "result copies");
+  // The copy of the error words costs about 8 us, more than a small call's
+  // kernels: it is made only when the device raised the flag.
+  if (!*err_flag_) return BINGO_OK;
   cuda_check(cudaMemcpy(h_err_, d_err_, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost), "read status");
   const uint32_t bits = h_err_[0], rejected = h_err_[1];
+  clear_err();
   if (!bits) return BINGO_OK;
-  cuda_check(cudaMemset(d_err_, 0, 2 * sizeof(uint32_t)), "clear status");
   const int st = status_of(bits);
   last_error = "device reported error bits 0x" + std::to_string(bits);
   if (bits & E_INVALID_SLOT) last_error += " (" + std::to_string(rejected) + " deletes of absent slots skipped)";
@@ -953,43 +968,61 @@ void Engine::finish_call() {
 }
 
 // ------------------------------------------------------------------ staging
+std::vector<Engine::Scratch> Engine::batch_scratch(uint64_t k) {
+  const uint64_t kk = std::max<uint64_t>(k, 1);
+  const uint64_t ks = std::max<uint64_t>(std::min<uint64_t>(kk, n_ ? n_ : kk), 1);
+  size_t t_sort = 0, t_sel = 0;
+  cub::DeviceRadixSort::SortPairs(nullptr, t_sort, (const uint32_t*)nullptr, (uint32_t*)nullptr,
+                                  (const uint32_t*)nullptr, (uint32_t*)nullptr, (int)kk, 0, 32, stream_);
+  cub::DeviceSelect::Flagged(nullptr, t_sel, (const uint32_t*)nullptr, (const uint8_t*)nullptr, (uint32_t*)nullptr,
+                             (uint32_t*)nullptr, (int)kk, stream_);
+  return {{&in_a_, kk * 4},
+          {&in_b_, kk * 4},
+          {&in_c_, kk * 4},
+          {&key_s_, kk * 4},
+          {&perm_, kk * 4},
+          {&sa_, kk * 4},
+          {&sb_, kk * 4},
+          {&head_, kk},
+          {&seg_, kk * 4},
+          {&slots_, kk * 4},
+          {&nseg_, 16},
+          {&ctl_, 16},
+          {&base_, kArenas * 8 * 2},
+          {&need_, (size_t)plan_blocks((uint32_t)ks) * sizeof(ArenaNeed)},  // plan-block sums
+          {&scan_, (size_t)ks * sizeof(ArenaNeed)},                         // in-block offsets
+          {&big_, (size_t)ks * 4},
+          {&cub_tmp_, std::max(t_sort, t_sel)},
+          {&iota_, kk * 4}};
+}
+
+void Engine::fill_iota(uint64_t k) {
+  k_iota<<<grid_for(k, kBlock), kBlock, 0, stream_>>>(iota_.as<uint32_t>(), k);
+  cuda_check(cudaGetLastError(), "iota");
+  ++launches_;
+  iota_n_ = k;
+}
+
 void Engine::ensure_batch_scratch(uint64_t k) {
   const uint64_t kk = std::max<uint64_t>(k, 1);
   if (slots_busy_ && slots_.bytes < kk * 4) {  // slots_ is about to move: its copy-out must be over
     cuda_check(cudaEventSynchronize(slots_ev_), "slot copy");
     slots_busy_ = false;
   }
-  const uint64_t ks = std::max<uint64_t>(std::min<uint64_t>(kk, n_ ? n_ : kk), 1);
-  in_a_.ensure(kk * 4, "scratch");
-  in_b_.ensure(kk * 4, "scratch");
-  in_c_.ensure(kk * 4, "scratch");
-  key_s_.ensure(kk * 4, "scratch");
-  perm_.ensure(kk * 4, "scratch");
-  sa_.ensure(kk * 4, "scratch");
-  sb_.ensure(kk * 4, "scratch");
-  head_.ensure(kk, "scratch");
-  seg_.ensure(kk * 4, "scratch");
-  slots_.ensure(kk * 4, "scratch");
-  nseg_.ensure(16, "scratch");
-  ctl_.ensure(16, "scratch");
-  base_.ensure(kArenas * 8 * 2, "scratch");
-  need_.ensure((size_t)plan_blocks((uint32_t)ks) * sizeof(ArenaNeed), "scratch");  // plan-block sums
-  scan_.ensure((size_t)ks * sizeof(ArenaNeed), "scratch");                                   // in-block offsets
-  big_.ensure((size_t)ks * 4, "scratch");
-  if (iota_n_ < kk) {
-    iota_.ensure(kk * 4, "scratch");
-    k_iota<<<grid_for(kk, kBlock), kBlock, 0, stream_>>>(iota_.as<uint32_t>(), kk);
-    cuda_check(cudaGetLastError(), "iota");
-    ++launches_;
-    iota_n_ = kk;
-  }
-  size_t t_sort = 0, t_sel = 0;
-  cub::DeviceRadixSort::SortPairs(nullptr, t_sort, (const uint32_t*)nullptr, (uint32_t*)nullptr,
-                                  (const uint32_t*)nullptr, (uint32_t*)nullptr, (int)kk, 0, 32, stream_);
-  cub::DeviceSelect::Flagged(nullptr, t_sel, (const uint32_t*)nullptr, (const uint8_t*)nullptr, (uint32_t*)nullptr,
-                             (uint32_t*)nullptr, (int)kk, stream_);
-  cub_tmp_.ensure(std::max(t_sort, t_sel), "scratch");
+  for (const Scratch& q : batch_scratch(k)) q.buf->ensure(q.bytes, "scratch");
+  if (iota_n_ < kk) fill_iota(kk);
   group_cluster_ok();  // probed here, outside any stream capture
+}
+
+// `slots` work counters of walk launches, two words each (next item, warps
+// done). Zeroed when allocated; every launch leaves its own zeroed.
+uint32_t* Engine::walk_queue(DevBuf& buf, size_t slots) {
+  const size_t want = slots * 8;
+  if (!buf.p || buf.bytes < want) {
+    buf.ensure(want, "walk queue");
+    cuda_check(cudaMemsetAsync(buf.p, 0, buf.bytes, stream_), "walk queue");
+  }
+  return buf.as<uint32_t>();
 }
 
 const uint32_t* Engine::stage(const uint32_t* p, uint64_t k, DevBuf& buf, const char* what) {
@@ -1104,13 +1137,22 @@ void Engine::grow_arena(int a, unsigned long long min_cap) {
   if (nc < min_cap)
     throw Error(BINGO_ERR_CAPACITY, std::string(kArenaName[a]) + " arena would exceed its 32-bit index range");
   const unsigned long long used = h_top_[a];
+  auto reserve = [&](DevBuf& b, size_t bytes) {  // the kept load scratch makes room when there is none
+    try {
+      b.ensure(bytes, "grow arena");
+    } catch (const Error& e) {
+      if (e.status != BINGO_ERR_CAPACITY || load_slab_in_use_ || !load_slab_.p) throw;
+      load_slab_.release();
+      b.ensure(bytes, "grow arena");
+    }
+  };
   DevBuf fresh;
-  fresh.ensure(nc * kUnitBytes[a], "grow arena");
+  reserve(fresh, nc * kUnitBytes[a]);
   if (used) cuda_check(cudaMemcpyAsync(fresh.p, arena_[a].p, used * kUnitBytes[a], cudaMemcpyDeviceToDevice, stream_),
                        "grow arena copy");
   if (a == A_MEMBER) {
     DevBuf fgs;
-    fgs.ensure(nc * 4, "grow arena");
+    reserve(fgs, nc * 4);
     if (used) cuda_check(cudaMemcpyAsync(fgs.p, gs_.p, used * 4, cudaMemcpyDeviceToDevice, stream_), "grow copy");
     cuda_check(cudaStreamSynchronize(stream_), "grow arena");
     gs_.release();
@@ -1125,23 +1167,52 @@ void Engine::grow_arena(int a, unsigned long long min_cap) {
   ++arena_gen_;
 }
 
+void Engine::drop_arenas() {
+  for (auto& a : arena_) a.release();
+  gs_.release();
+}
+
+namespace {
+// Whether a buffer kept from the graph before serves for `want` bytes: large
+// enough, and not so large that it holds memory others could use.
+bool fits(const DevBuf& b, size_t want) { return b.p && b.bytes >= want && b.bytes <= 2 * want + (1u << 20); }
+void refit(DevBuf& b, size_t want, const char* what) {
+  if (fits(b, want)) return;
+  b.release();
+  b.ensure(want, what);
+}
+}  // namespace
+
+// Arenas for a new graph. Those of the graph before are kept where they fit
+// (allocating and freeing them took most of a load: 18 of 27 ms for R-MAT
+// 20); when the device has no room beside them they are freed first.
 void Engine::alloc_arenas(const unsigned long long need[kArenas]) {
+  try {
+    size_arenas(need);
+  } catch (const Error& e) {
+    if (e.status != BINGO_ERR_CAPACITY) throw;
+    drop_arenas();
+    if (!load_slab_in_use_) load_slab_.release();
+    size_arenas(need);
+  }
+  cuda_check(cudaMemsetAsync(d_top_, 0, kArenas * sizeof(unsigned long long), stream_), "reset tops");
+  std::memset(h_top_, 0, kArenas * sizeof(unsigned long long));
+  ++arena_gen_;
+}
+
+void Engine::size_arenas(const unsigned long long need[kArenas]) {
   for (int a = 0; a < kArenas; ++a) {
     if (a == A_HASH && !cfg_.node2vec) {
       cap_[a] = 0;
-      arena_[a].ensure(256, "arena");
+      refit(arena_[a], 256, "arena");
       continue;
     }
     unsigned long long c = (unsigned long long)std::ceil((double)need[a] * cfg_.arena_factor);
     c = std::max(c, need[a] + kArenaFloor[a]);
     c = std::min(c, kArenaLimit[a]);
     if (c < need[a]) throw Error(BINGO_ERR_CAPACITY, std::string(kArenaName[a]) + " arena exceeds its index range");
-    arena_[a].release();
-    arena_[a].ensure(c * kUnitBytes[a], "allocate arena");
-    if (a == A_MEMBER) {
-      gs_.release();
-      gs_.ensure(c * 4, "allocate arena");
-    }
+    refit(arena_[a], c * kUnitBytes[a], "allocate arena");
+    if (a == A_MEMBER) refit(gs_, c * 4, "allocate arena");
     cap_[a] = c;
   }
   if (cfg_.arena_bytes) {
@@ -1154,9 +1225,6 @@ void Engine::alloc_arenas(const unsigned long long need[kArenas]) {
         if (cap_[a]) grow_arena(a, (unsigned long long)std::ceil(cap_[a] * scale));
     }
   }
-  cuda_check(cudaMemsetAsync(d_top_, 0, kArenas * sizeof(unsigned long long), stream_), "reset tops");
-  std::memset(h_top_, 0, kArenas * sizeof(unsigned long long));
-  ++arena_gen_;
 }
 
 // Per-segment arena offsets of the grouped insert batch relative to the
@@ -1232,7 +1300,7 @@ void Engine::run_insert(uint64_t k, uint32_t* dev_out_slots, bool load_mode, uin
     for (int a = 0; a < kArenas; ++a) h_top_[a] = h_plan_[kArenas + 1 + a];
   if (ctl) {
     cuda_check(cudaStreamSynchronize(stream_), "rejected batch");
-    cuda_check(cudaMemset(d_err_, 0, 2 * sizeof(uint32_t)), "clear status");
+    clear_err();
     const int st = status_of(ctl);
     throw Error(st, st == BINGO_ERR_ZERO_WEIGHT ? "batch holds a zero weight" : "batch holds a vertex id >= n");
   }
@@ -1274,19 +1342,29 @@ void Engine::load(const uint32_t* src, const uint32_t* dst, const uint32_t* w, u
   if (m && !is_device_ptr(src)) host_check_ids(src, m, n, "source");
   if (m && !is_device_ptr(dst)) host_check_ids(dst, m, n, "destination");
   if (m && !is_device_ptr(w)) host_check_weights(w, m);
-  cuda_check(cudaStreamSynchronize(stream_), "load");
+  // The buffers of the graph before are written again: all work on them must
+  // be over, whatever stream it was ordered on.
+  cuda_check(cudaDeviceSynchronize(), "load");
   loaded_ = false;
   n_ = n;
   ++arena_gen_;
-  vrec_.release(), meta_.release(), gdesc_.release();
-  vrec_.ensure((size_t)n * sizeof(VertexRec), "vertex records");
-  meta_.ensure((size_t)n * sizeof(VertexMeta), "vertex metadata");
-  gdesc_.ensure((size_t)n * kBits * sizeof(GroupDesc), "group descriptors");
+  for (int a = 0; a < kArenas; ++a) cap_[a] = 0;
+  try {
+    refit(vrec_, (size_t)n * sizeof(VertexRec), "vertex records");
+    refit(meta_, (size_t)n * sizeof(VertexMeta), "vertex metadata");
+    refit(gdesc_, (size_t)n * kBits * sizeof(GroupDesc), "group descriptors");
+  } catch (const Error& e) {
+    if (e.status != BINGO_ERR_CAPACITY) throw;
+    drop_arenas();
+    load_slab_.release();
+    vrec_.release(), meta_.release(), gdesc_.release();
+    vrec_.ensure((size_t)n * sizeof(VertexRec), "vertex records");
+    meta_.ensure((size_t)n * sizeof(VertexMeta), "vertex metadata");
+    gdesc_.ensure((size_t)n * kBits * sizeof(GroupDesc), "group descriptors");
+  }
   cuda_check(cudaMemsetAsync(vrec_.p, 0, (size_t)n * sizeof(VertexRec), stream_), "memset");
   cuda_check(cudaMemsetAsync(meta_.p, 0, (size_t)n * sizeof(VertexMeta), stream_), "memset");
   cuda_check(cudaMemsetAsync(gdesc_.p, 0, (size_t)n * kBits * sizeof(GroupDesc), stream_), "memset");
-  for (int a = 0; a < kArenas; ++a) arena_[a].release(), cap_[a] = 0;
-  gs_.release();
   cuda_check(cudaMemsetAsync(d_top_, 0, kArenas * sizeof(unsigned long long), stream_), "reset tops");
   std::memset(h_top_, 0, kArenas * sizeof(unsigned long long));
   if (m == 0) {
@@ -1296,20 +1374,74 @@ void Engine::load(const uint32_t* src, const uint32_t* dst, const uint32_t* w, u
     finish_call();
     return;
   }
-  ensure_batch_scratch(m);
-  const uint32_t* ds = stage(src, m, in_a_, "stage src");
-  const uint32_t* dd = stage(dst, m, in_b_, "stage dst");
-  const uint32_t* dw = stage(w, m, in_c_, "stage w");
-  group_by_vertex(ds, dd, dw, m, true);
-  run_insert(m, nullptr, true, m);
+  load_batch(src, dst, w, m);
   loaded_ = true;
-  // Release load-sized scratch; update batches re-grow what they need.
-  DevBuf* big[] = {&in_a_, &in_b_, &in_c_, &key_s_, &perm_, &sa_, &sb_, &head_, &seg_, &slots_, &need_,
-                   &scan_, &big_, &iota_, &cub_tmp_};
-  cuda_check(cudaStreamSynchronize(stream_), "load");
-  for (DevBuf* b : big) b->release();
-  iota_n_ = 0;
   finish_call();
+}
+
+// A load's batch, with its scratch in one slab (eighteen allocations and
+// frees of load size took 12 ms for R-MAT 20): the batch buffers point into
+// the slab meanwhile, and those that updates use come back after. The slab is
+// kept for the next load while it is small beside the graph.
+void Engine::load_batch(const uint32_t* src, const uint32_t* dst, const uint32_t* w, uint64_t m) {
+  if (slots_busy_) {
+    cuda_check(cudaEventSynchronize(slots_ev_), "slot copy");
+    slots_busy_ = false;
+  }
+  const std::vector<Scratch> need = batch_scratch(m);
+  size_t total = 0;
+  for (const Scratch& q : need) total += (q.bytes + 255) & ~(size_t)255;
+  try {
+    refit(load_slab_, total, "scratch");
+  } catch (const Error& e) {
+    if (e.status != BINGO_ERR_CAPACITY) throw;
+    drop_arenas();
+    for (const Scratch& q : need) q.buf->release();
+    iota_n_ = 0;
+    load_slab_.ensure(total, "scratch");
+  }
+  struct Borrow {  // the batch buffers point into the slab while this lives
+    Engine& e;
+    const std::vector<Scratch>& need;
+    std::vector<DevBuf> own;
+    uint64_t iota_n;
+    Borrow(Engine& e_, const std::vector<Scratch>& need_) : e(e_), need(need_), iota_n(e_.iota_n_) {
+      char* p = e.load_slab_.as<char>();
+      for (const Scratch& q : need) {
+        own.push_back(*q.buf);
+        q.buf->p = p, q.buf->bytes = q.bytes;
+        p += (q.bytes + 255) & ~(size_t)255;
+      }
+      e.load_slab_in_use_ = true;
+    }
+    ~Borrow() {
+      cudaStreamSynchronize(e.stream_);  // also after an error: nothing uses the slab past this
+      for (size_t i = 0; i < need.size(); ++i) *need[i].buf = own[i];
+      e.iota_n_ = iota_n;
+      e.load_slab_in_use_ = false;
+    }
+  };
+  {
+    Borrow borrow(*this, need);
+    group_cluster_ok();
+    fill_iota(m);
+    const uint32_t* ds = stage(src, m, in_a_, "stage src");
+    const uint32_t* dd = stage(dst, m, in_b_, "stage dst");
+    const uint32_t* dw = stage(w, m, in_c_, "stage w");
+    group_by_vertex(ds, dd, dw, m, true);
+    run_insert(m, nullptr, true, m);
+    cuda_check(cudaStreamSynchronize(stream_), "load");
+  }
+  size_t held = gs_.bytes + vrec_.bytes + meta_.bytes + gdesc_.bytes;
+  for (const auto& a : arena_) held += a.bytes;
+  const size_t keep = std::max<size_t>(held / 4, 64u << 20);
+  if (load_slab_.bytes > keep) load_slab_.release();
+  size_t own = 0;
+  for (const Scratch& q : need) own += q.buf->bytes;
+  if (own > keep) {  // of update batches before this load
+    for (const Scratch& q : need) q.buf->release();
+    iota_n_ = 0;
+  }
 }
 
 void Engine::insert(const uint32_t* src, const uint32_t* dst, const uint32_t* w, uint64_t k, uint32_t* out_slots) {
@@ -1390,7 +1522,7 @@ void Engine::check_batch_on_device(const uint32_t* a, const uint32_t* b, const u
   cuda_check(cudaMemcpyAsync(&ctl, ctl_.p, 4, cudaMemcpyDeviceToHost, stream_), "read ctl");
   cuda_check(cudaStreamSynchronize(stream_), "validate sync");
   if (ctl) {
-    cuda_check(cudaMemset(d_err_, 0, 2 * sizeof(uint32_t)), "clear status");
+    clear_err();
     const int st = status_of(ctl);
     throw Error(st, st == BINGO_ERR_ZERO_WEIGHT ? "batch holds a zero weight" : "batch holds a vertex id >= n");
   }
@@ -1600,14 +1732,12 @@ void Engine::walk(const bingo_walk_job* jobs, uint32_t n_jobs, uint32_t mode) {
       throw Error(BINGO_ERR_INVALID_ARGUMENT, "device output must be 32-byte aligned");
   }
   const WalkView W = wview();
-  queue_.ensure(4 * std::max<uint32_t>(n_jobs, 4), "walk queue");
-  uint32_t* q = queue_.as<uint32_t>();
+  uint32_t* q = walk_queue(queue_, std::max<uint32_t>(n_jobs, 4));
   if (mode == BINGO_WALK_PLAIN) {
     // One launch per job, each with its own work counter.
-    cuda_check(cudaMemsetAsync(q, 0, 4 * n_jobs, stream_), "queue reset");
     for (uint32_t j = 0; j < n_jobs; ++j) {
       if (!dj[j].n) continue;
-      launch_walk_job(stream_, W, dj[j], q + j, tuning_);
+      launch_walk_job(stream_, W, dj[j], q + 2 * j, tuning_);
       ++launches_;
     }
   } else if (prefix[n_jobs]) {
@@ -1622,11 +1752,10 @@ void Engine::walk(const bingo_walk_job* jobs, uint32_t n_jobs, uint32_t mode) {
                                stream_),
                "jobs H2D");
     cuda_check(cudaMemcpyAsync(prefix_.p, pf.data(), pf.size() * 4, cudaMemcpyHostToDevice, stream_), "prefix H2D");
-    cuda_check(cudaMemsetAsync(q, 0, 4 * groups.size(), stream_), "queue reset");
     for (size_t gi = 0; gi < groups.size(); ++gi) {
       const WalkGroup& G = groups[gi];
       launch_walk_table(stream_, G.app, W, table[G.job_off], jobs_.as<WalkJobDev>() + G.job_off,
-                        prefix_.as<uint32_t>() + G.pf_off, G.n_jobs, G.total, q + gi, tuning_);
+                        prefix_.as<uint32_t>() + G.pf_off, G.n_jobs, G.total, q + 2 * gi, tuning_);
       ++launches_;
     }
   }
@@ -1843,11 +1972,11 @@ void Engine::run(const bingo_op* ops, uint32_t n_ops, uint32_t flags) {
   // Job tables are read by the walk kernels from device memory, so their
   // contents may change between replays of a captured program.
   if (!table.empty()) {
-    const size_t jb = table.size() * sizeof(WalkJobDev), pb = pf.size() * 4, qb = groups.size() * 4;
+    const size_t jb = table.size() * sizeof(WalkJobDev), pb = pf.size() * 4, qb = groups.size() * 8;
     if (jb > prog_jobs_.bytes || pb > prog_prefix_.bytes || qb > prog_queue_.bytes) drop_graph();
     prog_jobs_.ensure(jb, "program jobs");
     prog_prefix_.ensure(pb, "program jobs");
-    prog_queue_.ensure(std::max<size_t>(qb, 4), "program queue");
+    walk_queue(prog_queue_, groups.size());
     cuda_check(cudaMemcpyAsync(prog_jobs_.p, table.data(), jb, cudaMemcpyHostToDevice, stream_), "program jobs H2D");
     cuda_check(cudaMemcpyAsync(prog_prefix_.p, pf.data(), pb, cudaMemcpyHostToDevice, stream_), "program jobs H2D");
   }
@@ -1857,8 +1986,6 @@ void Engine::run(const bingo_op* ops, uint32_t n_ops, uint32_t flags) {
 
   const uint64_t launches0 = launches_;
   auto enqueue_all = [&]() {
-    if (!groups.empty())
-      cuda_check(cudaMemsetAsync(prog_queue_.p, 0, groups.size() * 4, stream_), "program queue reset");
     const WalkView W = wview();
     for (uint32_t i = 0; i < n_ops; ++i) {
       const bingo_op& o = ops[i];
@@ -1874,7 +2001,7 @@ void Engine::run(const bingo_op* ops, uint32_t n_ops, uint32_t flags) {
           const WalkGroup& G = groups[gi];
           launch_walk_table(stream_, G.app, W, table[G.job_off], prog_jobs_.as<WalkJobDev>() + G.job_off,
                             prog_prefix_.as<uint32_t>() + G.pf_off, G.n_jobs, G.total,
-                            prog_queue_.as<uint32_t>() + gi, tuning_);
+                            prog_queue_.as<uint32_t>() + 2 * gi, tuning_);
           ++launches_;
         }
       }
@@ -1920,7 +2047,7 @@ constexpr uint32_t kNoAllocMaxJobs = 64;
 struct NoAllocScratch {
   WalkJobDev jobs[kNoAllocMaxJobs];
   uint32_t prefix[kNoAllocMaxJobs + 1];
-  uint32_t queue;
+  uint32_t queue[2];
 };
 static __device__ __align__(256) unsigned char g_noalloc_scratch[sizeof(NoAllocScratch)];
 
@@ -1941,7 +2068,7 @@ __global__ void k_noalloc_stage(const __grid_constant__ NoAllocJobs in, NoAllocS
   uint32_t* out = reinterpret_cast<uint32_t*>(dst->jobs);
   for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) out[i] = src[i];
   for (uint32_t i = threadIdx.x; i <= in.n_jobs; i += blockDim.x) dst->prefix[i] = in.prefix[i];
-  if (threadIdx.x == 0) dst->queue = 0;
+  if (threadIdx.x == 0) dst->queue[0] = dst->queue[1] = 0;
 }
 static_assert(sizeof(WalkJobDev) % 4 == 0, "word copy");
 
@@ -2024,7 +2151,7 @@ void Engine::walk_noalloc(const bingo_walk_job* jobs, uint32_t n_jobs) {
   cuda_check(cudaGetLastError(), "no-alloc job staging");
   ++launches_;
   const WalkView W = wview();
-  launch_walk_table(stream_, -1, W, dj[0], scratch->jobs, scratch->prefix, n_jobs, (uint32_t)total, &scratch->queue,
+  launch_walk_table(stream_, -1, W, dj[0], scratch->jobs, scratch->prefix, n_jobs, (uint32_t)total, scratch->queue,
                     tuning_);
   ++launches_;
   finish_call();
@@ -2078,7 +2205,7 @@ void Engine::stats(bingo_stats* out) {
   const DevBuf* sc[] = {&in_a_, &in_b_, &in_c_, &key_s_, &perm_, &iota_, &sa_, &sb_, &head_, &seg_, &nseg_,
                         &need_, &scan_, &big_, &base_, &ctl_, &slots_, &cub_tmp_, &jobs_, &prefix_, &queue_, &wstart_,
                         &wout_[0], &wout_[1], &pair_key_, &pair_key_s_, &pair_slot_, &fw_in_, &fw_fixed_,
-                        &prog_jobs_, &prog_prefix_, &prog_queue_};
+                        &prog_jobs_, &prog_prefix_, &prog_queue_, &load_slab_};
   for (const DevBuf* b : sc) out->scratch_bytes += b->bytes;
 }
 
@@ -2270,8 +2397,8 @@ void Engine::restore_state(const StateCopy& c) {
     cuda_check(cudaMemcpyAsync(gs_.p, c.gs.p, c.top[A_MEMBER] * 4, cudaMemcpyDeviceToDevice, stream_), "state restore");
   cuda_check(cudaMemcpyAsync(d_top_, h_top_, kArenas * sizeof(unsigned long long), cudaMemcpyHostToDevice, stream_),
              "state restore");
-  cuda_check(cudaMemsetAsync(d_err_, 0, 2 * sizeof(uint32_t), stream_), "state restore");
   cuda_check(cudaStreamSynchronize(stream_), "state restore");
+  clear_err();
 }
 
 // ------------------------------------------------------------------ snapshot files
@@ -2483,7 +2610,8 @@ void Engine::restore(const char* path) {
   for (int a = 0; a < kArenas; ++a) h_top_[a] = H.top[a];
   cuda_check(cudaMemcpyAsync(d_top_, h_top_, kArenas * sizeof(unsigned long long), cudaMemcpyHostToDevice, stream_),
              "restore");
-  cuda_check(cudaMemsetAsync(d_err_, 0, 2 * sizeof(uint32_t), stream_), "restore");
+  cuda_check(cudaStreamSynchronize(stream_), "restore");
+  clear_err();
   // The checksum only shows the file is the one written; the store check
   // shows its content is a store the kernels can index safely.
   bingo_check_report rep{};

@@ -133,7 +133,8 @@ class Engine {
   unsigned long long* d_top_ = nullptr;  // [kArenas]
   unsigned long long cap_[kArenas] = {};
   uint32_t* d_err_ = nullptr;            // [0] ErrBit sticky, [1] rejected deletes
-  uint32_t* h_err_ = nullptr;            // pinned mirror
+  uint32_t* h_err_ = nullptr;            // pinned mirror of its first two words
+  volatile unsigned long long* err_flag_ = nullptr;  // raised by the device with an error (in h_plan_'s block)
   unsigned long long* h_top_ = nullptr;  // pinned mirror of d_top_
   // Insert plan read-back (totals, status, tops) through mapped host memory,
   // written by a kernel: no copy-engine transfer that could queue behind a
@@ -148,6 +149,8 @@ class Engine {
   // per-batch scratch
   DevBuf in_a_, in_b_, in_c_, key_s_, perm_, iota_, sa_, sb_, head_, seg_, nseg_, need_, scan_, big_, base_, ctl_,
       slots_, cub_tmp_;
+  DevBuf load_slab_;                          // a load's scratch, kept for the next one
+  bool load_slab_in_use_ = false;
   DevBuf pair_key_, pair_key_s_, pair_slot_;  // delete-by-pair translation
   DevBuf fw_in_, fw_fixed_;                   // float weights: staged input, 16.16 fixed point
   DevBuf check_buf_, check_big_;              // store check: totals, large-vertex list
@@ -174,7 +177,18 @@ class Engine {
 
   StoreView view() const;
   WalkView wview() const;
+  void clear_err();
+  struct Scratch {
+    DevBuf* buf;
+    size_t bytes;
+  };
+  std::vector<Scratch> batch_scratch(uint64_t k);  // what a batch of k edges needs
   void ensure_batch_scratch(uint64_t k);
+  void fill_iota(uint64_t k);
+  void load_batch(const uint32_t* src, const uint32_t* dst, const uint32_t* w, uint64_t m);
+  void drop_arenas();
+  void size_arenas(const unsigned long long need[kArenas]);
+  uint32_t* walk_queue(DevBuf& buf, size_t slots);  // zeroed work counters
   const uint32_t* stage(const uint32_t* p, uint64_t k, DevBuf& buf, const char* what);
   // Stable grouping of a batch by `key` into key_s_/perm_/sa_/sb_/seg_/nseg_,
   // with the batch status word zeroed and the batch validated (`insert`: the

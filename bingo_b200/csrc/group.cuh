@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
   bits = __reduce_or_sync(kFull, bits);
   if (bits && l == 0) {
     atomicOr(ctl, bits);
-    atomicOr(err, bits);
+    set_err(err, bits);
   }
   cluster.sync();  // no CTA exits while another may still read its shared memory
 }
