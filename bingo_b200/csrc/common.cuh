@@ -127,6 +127,8 @@ __device__ __forceinline__ unsigned long long mulhi64(unsigned long long a, unsi
   return __umul64hi(a, b);
 }
 
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 __device__ __forceinline__ uint32_t lanemask_lt() {
   uint32_t m;
   asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));

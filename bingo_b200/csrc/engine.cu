@@ -120,11 +120,6 @@ __device__ __forceinline__ void seg_bounds(const uint32_t* seg, uint32_t S, uint
   *e = s + 1 < S ? seg[s + 1] : (uint32_t)k;
 }
 
-// Arena sizes one segment needs (units of each arena).
-struct ArenaNeed {
-  unsigned long long v[kArenas];
-};
-
 // Plan blocks: one segment per warp, kPlanSegs consecutive segments per block.
 constexpr int kPlanThreads = 1024;
 constexpr int kPlanSegs = kPlanThreads / 32;
@@ -344,12 +339,19 @@ struct HostReserve {
 
 
 
-__global__ void __launch_bounds__(kBlock, 4) k_apply_insert(StoreView S, const uint32_t* skey, const uint32_t* sv,
+// Consecutive segments a warp of the apply kernels takes at a time: their
+// bounds, and what a delete needs first, are read for all of them at once.
+__device__ __forceinline__ uint32_t segs_per_warp(uint32_t nS, uint32_t warps) {
+  return min(8u, max(1u, nS / warps));
+}
+
+__global__ void __launch_bounds__(kBlock, 4) k_apply_insert(const __grid_constant__ StoreView S, const uint32_t* skey, const uint32_t* sv,
                                                          const uint32_t* sw, const uint32_t* sorig,
                                                          const uint32_t* seg, const uint32_t* nseg,
                                                          unsigned long long k, uint32_t ks, const uint32_t* ctl,
                                                          const ArenaNeed* excl, const unsigned long long* boff,
-                                                         const unsigned long long* base, HostReserve hr,
+                                                         const unsigned long long* base,
+                                                         const __grid_constant__ HostReserve hr,
                                                          const uint32_t* big, uint32_t* out_slots) {
   static_assert(kBlock / 32 == kAppendWarps, "a block appends a listed segment");
   pdl_wait();
@@ -367,47 +369,101 @@ __global__ void __launch_bounds__(kBlock, 4) k_apply_insert(StoreView S, const u
     const uint32_t s = big[q];
     uint32_t b, e;
     seg_bounds(seg, nS, s, k, &b, &e);
-    unsigned long long res[kArenas];
-    for (int a = 0; a < kArenas; ++a)
-      res[a] = (base ? base[a] : hr.base[a]) + boff[(size_t)a * nb + s / kPlanSegs] + (excl[s].v[a] & ~kBigFlag);
-    apply_append_block(S, skey[b], sv + b, sw + b, sorig + b, e - b, out_slots, res, &asc[threadIdx.x / 32], ba);
-  }
-  // The other segments, one warp each; blocks that had a listed one leave them
-  // to the rest while those are the most.
-  const uint32_t skip = nbig < gridDim.x / 2 ? nbig : 0u;
-  if (blockIdx.x < skip) return;
-  const uint32_t warps = (gridDim.x - skip) * (blockDim.x / 32);
-  for (uint32_t s = ((blockIdx.x - skip) * blockDim.x + threadIdx.x) / 32; s < nS; s += warps) {
-    uint32_t b, e;
-    seg_bounds(seg, nS, s, k, &b, &e);
-    const uint32_t u = skey[b];
-    if (u >= S.n) continue;
-    const ArenaNeed off = excl[s];
-    if (off.v[A_EDGE] & kBigFlag) continue;
-    unsigned long long res[kArenas];
+    ArenaNeed res;
 #pragma unroll
     for (int a = 0; a < kArenas; ++a)
-      res[a] = (base ? base[a] : hr.base[a]) + boff[(size_t)a * nb + s / kPlanSegs] + off.v[a];
-    apply_append(S, u, sv + b, sw + b, sorig + b, e - b, out_slots, res, &asc[threadIdx.x / 32]);
+      res.v[a] = (base ? base[a] : hr.base[a]) + boff[(size_t)a * nb + s / kPlanSegs] + (excl[s].v[a] & ~kBigFlag);
+    apply_append_block(S, skey[b], sv + b, sw + b, sorig + b, e - b, out_slots, res, asc[threadIdx.x / 32], ba);
+  }
+  // The other segments, one warp each, `per` consecutive ones at a time;
+  // blocks that had a listed one leave them to the rest while those are the
+  // most.
+  const uint32_t skip = nbig < gridDim.x / 2 ? nbig : 0u;
+  if (blockIdx.x < skip) return;
+  const int lane = threadIdx.x & 31;
+  AliasScratch& A = asc[threadIdx.x / 32];
+  const uint32_t warps = (gridDim.x - skip) * (kBlock / 32), per = segs_per_warp(nS, warps);
+  for (uint32_t s0 = ((blockIdx.x - skip) * kBlock + threadIdx.x) / 32 * per; s0 < nS; s0 += warps * per) {
+    // Lane i: segment s0 + i.
+    const uint32_t s = s0 + lane;
+    uint32_t b = 0, e = 0, u = 0xffffffffu;
+    if (lane < (int)per && s < nS) {
+      seg_bounds(seg, nS, s, k, &b, &e);
+      u = skey[b];
+      if (excl[s].v[A_EDGE] & kBigFlag) u = 0xffffffffu;
+    }
+    for (uint32_t todo = __ballot_sync(kFull, u < S.n); todo; todo &= todo - 1) {
+      const int src = __ffs(todo) - 1;
+      const uint32_t vb = __shfl_sync(kFull, b, src), ve = __shfl_sync(kFull, e, src), vs = s0 + src;
+      auto res = [&](int a) {
+        return (base ? base[a] : hr.base[a]) + boff[(size_t)a * nb + vs / kPlanSegs] + (excl[vs].v[a] & ~kBigFlag);
+      };
+      apply_append(S, __shfl_sync(kFull, u, src), sv + vb, sw + vb, sorig + vb, ve - vb, out_slots, res, A);
+    }
   }
 }
 
-__global__ void __launch_bounds__(kBlock, 3) k_apply_delete(StoreView S, const uint32_t* skey, const uint32_t* sslot,
+__global__ void __launch_bounds__(kBlock, 4) k_apply_delete(const __grid_constant__ StoreView S, const uint32_t* skey, const uint32_t* sslot,
                                                          const uint32_t* seg, const uint32_t* nseg,
                                                          unsigned long long k, const uint32_t* ctl) {
   pdl_wait();
   pdl_trigger();
+  static_assert(kBlock / 32 == kDeleteWarps, "a block deletes a long segment");
   __shared__ AliasScratch asc[kBlock / 32];
   __shared__ uint32_t stage[kBlock / 32][64];
+  __shared__ BlockDelete bd;
+  __shared__ uint32_t llist[kBlock], nlong;
   if (*ctl) return;
-  const uint32_t warps = gridDim.x * blockDim.x / 32;
   const uint32_t nS = *nseg;
-  for (uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) / 32; s < nS; s += warps) {
+  // Long segments, a block each: every block looks through its share (spread,
+  // since the hubs of a skewed graph are neighbours).
+  for (uint32_t t0 = 0; t0 < nS; t0 += gridDim.x * kBlock) {
+    if (threadIdx.x == 0) nlong = 0;
+    __syncthreads();
+    const uint32_t s = t0 + blockIdx.x + gridDim.x * threadIdx.x;
     uint32_t b, e;
-    seg_bounds(seg, nS, s, k, &b, &e);
-    const uint32_t u = skey[b];
-    if (u >= S.n) continue;
-    apply_delete(S, u, sslot + b, e - b, stage[threadIdx.x / 32], &asc[threadIdx.x / 32]);
+    if (s < nS) {
+      seg_bounds(seg, nS, s, k, &b, &e);
+      if (e - b > kBigDelete && skey[b] < S.n) llist[atomicAdd(&nlong, 1u)] = s;
+    }
+    __syncthreads();
+    for (uint32_t q = 0; q < nlong; ++q) {
+      seg_bounds(seg, nS, llist[q], k, &b, &e);
+      apply_delete_block(S, skey[b], sslot + b, e - b, asc[threadIdx.x / 32], bd);
+    }
+    __syncthreads();
+  }
+  // The others, as in k_apply_insert.
+  const int lane = threadIdx.x & 31;
+  AliasScratch& A = asc[threadIdx.x / 32];
+  const uint32_t warps = gridDim.x * (kBlock / 32), per = segs_per_warp(nS, warps);
+  for (uint32_t s0 = (blockIdx.x * kBlock + threadIdx.x) / 32 * per; s0 < nS; s0 += warps * per) {
+    const uint32_t s = s0 + lane;
+    uint32_t b = 0, e = 0, u = 0xffffffffu;
+    if (lane < (int)per && s < nS) {
+      seg_bounds(seg, nS, s, k, &b, &e);
+      u = skey[b];
+    }
+    // The vertices' records and their first deletes' slots and back-pointers
+    // are brought near for all of them at once: each would be a chain of
+    // three reads from DRAM in its turn.
+    if (u < S.n) {
+      const VertexMeta* const M = S.meta + u;
+      const uint32_t slot = sslot[b];
+      prefetch_l2(S.gdesc + (size_t)u * kBits);
+      prefetch_l2(S.gdesc + (size_t)u * kBits + kBits / 2);
+      prefetch_l2(S.vrec + u);
+      if (slot < M->ecnt) {
+        const uint32_t ebp = S.edges[M->eoff + slot].ebp;
+        prefetch_l2(S.bp + M->bpoff + ebp);
+        prefetch_l2(S.bp + M->bpoff + ebp + 7);
+      }
+    }
+    for (uint32_t todo = __ballot_sync(kFull, u < S.n && e - b <= kBigDelete); todo; todo &= todo - 1) {
+      const int src = __ffs(todo) - 1;
+      const uint32_t vb = __shfl_sync(kFull, b, src), ve = __shfl_sync(kFull, e, src);
+      apply_delete(S, __shfl_sync(kFull, u, src), sslot + vb, ve - vb, stage[threadIdx.x / 32], A);
+    }
   }
 }
 

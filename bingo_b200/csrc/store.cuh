@@ -177,6 +177,11 @@ __device__ __forceinline__ bool hash_has(const HashEntry* tab, uint32_t hmask, u
   return h >= 0 && __ldg(&tab[h].cnt) > 0;
 }
 
+// Arena sizes one segment needs (units of each arena).
+struct ArenaNeed {
+  unsigned long long v[kArenas];
+};
+
 // ---------------------------------------------------------------------------
 // Growth plan for appending `len` edges to a vertex. All lanes compute the
 // same values; lane k also knows whether group k grows and to what capacity.
@@ -322,6 +327,7 @@ __device__ __forceinline__ void append_range(const StoreView& S, const VertexMet
 // (Lines: a warp takes about 3 us per 32 edges and a block 10 us to share a
 // segment out. Measured, R-MAT 20: load apply 6.9 ms to 2.9; 50K-edge insert
 // batches whose vertices follow the degree, 130 us to 79.)
+constexpr uint32_t kLaneCopy = 8;          // members of a moving list that one lane copies
 constexpr uint32_t kBigLen = 256;          // edges
 constexpr uint32_t kBigCopy = 1024;        // 16-byte units copied by relocations
 constexpr unsigned long long kBigFlag = 1ull << 63;  // marks such a segment in its A_EDGE offset
@@ -329,16 +335,17 @@ constexpr unsigned long long kBigFlag = 1ull << 63;  // marks such a segment in 
 // ---------------------------------------------------------------------------
 // Apply a growth plan (relocations drawn from per-arena bases reserved for
 // this segment), append the segment's edges in order, refresh the adjacency
-// index and rebuild the alias table. Replaces NodeData::copy / insert /
+// index and stage the alias table (alias_finish writes it). Replaces NodeData::copy / insert /
 // buildAliasTable (include/Bingo.cuh:95-110, :182-198, :111-158) and the host
 // reMalloc round trip (include/operation.cuh:163-174).
 //
 // seg_v / seg_w / seg_orig: the segment's edges in batch order; out_slots is
-// indexed by seg_orig (may be null). res[a]: the arena offsets reserved for
-// this segment (units of each arena).
-static __device__ void apply_append(const StoreView& S, uint32_t u, const uint32_t* seg_v, const uint32_t* seg_w,
+// indexed by seg_orig (may be null). res(a): the arena offset reserved for
+// this segment (units of each arena), read where a relocation needs it.
+template <class Reserved>
+static __device__ __forceinline__ void apply_append(const StoreView& S, uint32_t u, const uint32_t* seg_v, const uint32_t* seg_w,
                              const uint32_t* seg_orig, uint32_t len, uint32_t* out_slots,
-                             const unsigned long long res[kArenas], AliasScratch* sc) {
+                             const Reserved& res, AliasScratch& B) {
   const int lane = threadIdx.x & 31;
   VertexMeta M = S.meta[u];
   GroupDesc G = S.gdesc[(size_t)u * kBits + lane];
@@ -354,25 +361,41 @@ static __device__ void apply_append(const StoreView& S, uint32_t u, const uint32
 
   // --- relocations (old contents keep their order) ---
   if (P.new_ecap) {
-    warp_copy_v4(reinterpret_cast<uint4*>(S.edges + res[A_EDGE]), reinterpret_cast<const uint4*>(S.edges + M.eoff),
+    warp_copy_v4(reinterpret_cast<uint4*>(S.edges + res(A_EDGE)), reinterpret_cast<const uint4*>(S.edges + M.eoff),
                  M.ecnt, lane);
-    M.eoff = res[A_EDGE];
+    M.eoff = res(A_EDGE);
     M.ecap = P.new_ecap;
   }
   if (P.new_bpcap) {
-    warp_copy_u32(S.bp + res[A_BP], S.bp + M.bpoff, M.bpcnt, lane);
-    M.bpoff = res[A_BP];
+    warp_copy_u32(S.bp + res(A_BP), S.bp + M.bpoff, M.bpcnt, lane);
+    M.bpoff = res(A_BP);
     M.bpcap = P.new_bpcap;
   }
   {
-    // Lists that move: the whole warp copies the members of each non-empty
-    // one in turn; every moving lane then takes its new base (a list that
-    // held no members needs no copy, the common case for a new group).
+    // Lists that move: each lane copies its own when it is short, all lanes'
+    // reads in flight together (most moving lists hold 4 or 8 members); the
+    // whole warp copies the longer ones in turn. A list that held no members
+    // needs no copy (the common case for a new group).
     const uint32_t old_base = group_base(G);
-    uint32_t copy = __ballot_sync(kFull, P.gcap_lane != 0 && G.cnt != 0);
-    if (P.gcap_lane) {
-      G.base1 = (uint32_t)((res[A_MEMBER] + P.gpre) >> 2) + 1u;  // reserved offsets are 4-entry aligned
+    const bool moves = P.gcap_lane != 0;
+    const unsigned long long fresh = __any_sync(kFull, moves) ? res(A_MEMBER) : 0ull;
+    uint32_t copy = __ballot_sync(kFull, moves && G.cnt > kLaneCopy);
+    if (moves) {
+      G.base1 = (uint32_t)((fresh + P.gpre) >> 2) + 1u;  // reserved offsets are 4-entry aligned
       G.roomy = 0;
+      if (G.cnt <= kLaneCopy) {
+        const uint4* const v0 = reinterpret_cast<const uint4*>(S.gv) + old_base;
+        const uint4* const s0 = reinterpret_cast<const uint4*>(S.gs) + old_base;
+        uint4* const v1 = reinterpret_cast<uint4*>(S.gv) + group_base(G);
+        uint4* const s1 = reinterpret_cast<uint4*>(S.gs) + group_base(G);
+        uint4 a[2], b[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+          if (4u * q < G.cnt) a[q] = v0[q], b[q] = s0[q];
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+          if (4u * q < G.cnt) v1[q] = a[q], s1[q] = b[q];
+      }
     }
     while (copy) {
       const int k = __ffs(copy) - 1;
@@ -384,7 +407,7 @@ static __device__ void apply_append(const StoreView& S, uint32_t u, const uint32
     }
   }
   if (P.new_acap) {
-    R.aoff = (uint32_t)res[A_ALIAS];
+    R.aoff = (uint32_t)res(A_ALIAS);
     M.acap = P.new_acap;
   }
   __syncwarp();
@@ -423,7 +446,7 @@ static __device__ void apply_append(const StoreView& S, uint32_t u, const uint32
     if (P.rehash) {
       // Rebuild from every live slot into a cleared table.
       if (P.new_hcap) {
-        R.hoff = (uint32_t)res[A_HASH];
+        R.hoff = (uint32_t)res(A_HASH);
         R.hmask = P.new_hcap - 1;
         M.hcap = P.new_hcap;
       }
@@ -443,7 +466,7 @@ static __device__ void apply_append(const StoreView& S, uint32_t u, const uint32
   __syncwarp();
 
   // --- alias table over the new counts ---
-  R.m = warp_build_alias(lane, G.cnt, group_base(G), single, S.alias + R.aoff, sc);
+  R.m = warp_build_alias(lane, G.cnt, group_base(G), single, S.alias + R.aoff, &B);
   if (add_lane && !P.gcap_lane) G.roomy = group_roomy(G.cnt, cap0);
   if (add_lane || P.gcap_lane) S.gdesc[(size_t)u * kBits + lane] = G;  // only the descriptors that changed
   if (lane == 0) {
@@ -481,8 +504,8 @@ struct BlockAppend {
 // the adjacency updates. The store is the one apply_append leaves.
 static __device__ __noinline__ void apply_append_block(const StoreView& S, uint32_t u, const uint32_t* seg_v,
                                                        const uint32_t* seg_w, const uint32_t* seg_orig, uint32_t len,
-                                                       uint32_t* out_slots, const unsigned long long res[kArenas],
-                                                       AliasScratch* sc, BlockAppend& B) {
+                                                       uint32_t* out_slots, ArenaNeed at, AliasScratch& A,
+                                                       BlockAppend& B) {
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
   VertexMeta M = S.meta[u];
   GroupDesc G = S.gdesc[(size_t)u * kBits + lane];
@@ -510,21 +533,21 @@ static __device__ __noinline__ void apply_append_block(const StoreView& S, uint3
   const GrowPlan P = plan_growth(lane, M, G, len, add_lane, pc_total, S.node2vec);
   // --- relocations (old contents keep their order) ---
   if (P.new_ecap) {
-    block_copy_v4(reinterpret_cast<uint4*>(S.edges + res[A_EDGE]), reinterpret_cast<const uint4*>(S.edges + M.eoff),
+    block_copy_v4(reinterpret_cast<uint4*>(S.edges + at.v[A_EDGE]), reinterpret_cast<const uint4*>(S.edges + M.eoff),
                   M.ecnt);
-    M.eoff = res[A_EDGE];
+    M.eoff = at.v[A_EDGE];
     M.ecap = P.new_ecap;
   }
   if (P.new_bpcap) {
-    block_copy_u32(S.bp + res[A_BP], S.bp + M.bpoff, M.bpcnt);
-    M.bpoff = res[A_BP];
+    block_copy_u32(S.bp + at.v[A_BP], S.bp + M.bpoff, M.bpcnt);
+    M.bpoff = at.v[A_BP];
     M.bpcap = P.new_bpcap;
   }
   {
     const uint32_t old_base = group_base(G);
     uint32_t copy = __ballot_sync(kFull, P.gcap_lane != 0 && G.cnt != 0);
     if (P.gcap_lane) {
-      G.base1 = (uint32_t)((res[A_MEMBER] + P.gpre) >> 2) + 1u;
+      G.base1 = (uint32_t)((at.v[A_MEMBER] + P.gpre) >> 2) + 1u;
       G.roomy = 0;
     }
     while (copy) {  // the same lists in every warp
@@ -537,11 +560,11 @@ static __device__ __noinline__ void apply_append_block(const StoreView& S, uint3
     }
   }
   if (P.new_acap) {
-    R.aoff = (uint32_t)res[A_ALIAS];
+    R.aoff = (uint32_t)at.v[A_ALIAS];
     M.acap = P.new_acap;
   }
   if (P.new_hcap) {
-    R.hoff = (uint32_t)res[A_HASH];
+    R.hoff = (uint32_t)at.v[A_HASH];
     R.hmask = P.new_hcap - 1;
     M.hcap = P.new_hcap;
   }
@@ -581,7 +604,7 @@ static __device__ __noinline__ void apply_append_block(const StoreView& S, uint3
   // --- alias table over the new counts ---
   if (wi == 0) {
     G.cnt = cnt0 + add_lane;
-    R.m = warp_build_alias(lane, G.cnt, group_base(G), B.single[lane], S.alias + R.aoff, sc);
+    R.m = warp_build_alias(lane, G.cnt, group_base(G), B.single[lane], S.alias + R.aoff, &A);
     if (add_lane && !P.gcap_lane) G.roomy = group_roomy(G.cnt, cap0);
     if (add_lane || P.gcap_lane) S.gdesc[(size_t)u * kBits + lane] = G;
     if (lane == 0) {
@@ -611,8 +634,11 @@ __device__ __forceinline__ bool plan_append(const StoreView& S, uint32_t u, uint
   return len > kBigLen || moved > kBigCopy;
 }
 
-// Removals of one group a lane resolves per round of loads (apply_delete).
-constexpr int kDeleteRound = 4;
+// Removals of one group a lane resolves per round of loads (apply_delete; a
+// block takes the segments with many). Two keep the kernel at 64 registers and
+// four blocks per SM: 500K deletes 509 us against 532 at four removals and
+// three blocks.
+constexpr int kDeleteRound = 2;
 
 // ---------------------------------------------------------------------------
 // Delete a run of slots of one vertex in batch order. Each delete swap-removes
@@ -627,7 +653,7 @@ constexpr int kDeleteRound = 4;
 // (include/Bingo.cuh:199-218) and deleteKernel (include/operation.cuh:198-214).
 // stage: 64 words of shared memory owned by this warp.
 static __device__ void apply_delete(const StoreView& S, uint32_t u, const uint32_t* seg_slot, uint32_t len,
-                                    uint32_t* stage, AliasScratch* sc) {
+                                    uint32_t* stage, AliasScratch& B) {
   const int lane = threadIdx.x & 31;
   const uint32_t below = lanemask_lt();
   VertexMeta M = S.meta[u];
@@ -635,6 +661,50 @@ static __device__ void apply_delete(const StoreView& S, uint32_t u, const uint32
   VertexRec R = S.vrec[u];
   const size_t gb = (size_t)group_base(G) * 4;
   const uint32_t cnt0 = G.cnt, cap0 = group_cap(G);
+  if (len == 1) {
+    // One delete: lane k swap-removes its member when the weight has bit k.
+    const uint32_t slot = seg_slot[0];
+    EdgeRec e{0, 0, 0, 0};
+    if (slot < M.ecnt) e = S.edges[M.eoff + slot];
+    uint32_t single = 0;
+    if (e.w) {
+      const bool has = (e.w >> lane) & 1u;
+      const uint32_t c0 = G.cnt;
+      uint32_t pos = 0, tv = 0, tbi = 0;
+      if (has) {
+        pos = S.bp[M.bpoff + e.ebp + __popc(e.w & below)];
+        tv = S.gv[gb + c0 - 1];
+        tbi = S.gs[gb + c0 - 1];
+      }
+      // A group left with one member is named by it in the alias table.
+      if (has ? c0 == 2 : c0 == 1) single = S.gv[gb];
+      if (has) {
+        if (pos != c0 - 1) {
+          S.gv[gb + pos] = tv;
+          S.gs[gb + pos] = tbi;
+          S.bp[M.bpoff + tbi] = pos;
+          if (pos == 0) single = tv;
+        }
+        G.cnt = c0 - 1;
+        G.roomy = group_roomy(c0 - 1, cap0);
+        S.gdesc[(size_t)u * kBits + lane] = G;
+      }
+      if (lane == 0) {
+        S.edges[M.eoff + slot].w = 0u;
+        if (S.node2vec && R.hmask) hash_sub(S.hash + R.hoff, R.hmask, e.v, e.w);
+        S.meta[u].live = M.live - 1;
+      }
+    } else {
+      single = G.cnt == 1 ? S.gv[gb] : 0u;
+      if (lane == 0) {
+        atomicAdd(&S.err[1], 1u);
+        set_err(S.err, E_INVALID_SLOT);
+      }
+    }
+    const uint32_t m = warp_build_alias(lane, G.cnt, group_base(G), single, S.alias + R.aoff, &B);
+    if (lane == 0 && m != R.m) S.vrec[u].m = m;
+    return;
+  }
   uint32_t rejected = 0;
   bool front_known = false;  // this lane moved a member into position 0
   uint32_t front = 0;
@@ -722,7 +792,7 @@ static __device__ void apply_delete(const StoreView& S, uint32_t u, const uint32
   }
   // A group left with one member is named by it in the alias table.
   const uint32_t single = G.cnt == 1 ? (front_known ? front : S.gv[gb]) : 0u;
-  R.m = warp_build_alias(lane, G.cnt, group_base(G), single, S.alias + R.aoff, sc);
+  R.m = warp_build_alias(lane, G.cnt, group_base(G), single, S.alias + R.aoff, &B);
   if (G.cnt != cnt0) {  // only the descriptors that changed
     G.roomy = group_roomy(G.cnt, cap0);
     S.gdesc[(size_t)u * kBits + lane] = G;
@@ -731,6 +801,115 @@ static __device__ void apply_delete(const StoreView& S, uint32_t u, const uint32
     S.meta[u] = M;
     S.vrec[u] = R;
   }
+}
+
+// Segments a whole block deletes (apply_delete_block): a warp's lane resolves
+// the removals of its group a few per round trip, so a hub's deletes were a
+// chain that set the kernel's time (50K deletes on R-MAT 20: 116 of vertex 0,
+// 55 of them in one group; 500K: over a thousand). 500K deletes with the
+// grouping: 632 us, 509 with this and the reads below brought near.
+constexpr uint32_t kBigDelete = 24;
+
+constexpr int kDeleteWarps = 8;  // warps of a block that deletes one segment
+struct BlockDelete {
+  uint32_t w[32], ebp[32];          // the chunk's slots: weight (0 = skipped), back-pointer run
+  uint32_t order[kDeleteWarps][32]; // a warp's removals of one group, as back-pointer indices
+  uint32_t cnt[kBits];              // group counts at the end
+};
+
+// apply_delete by a block of kDeleteWarps warps, 32 deletes at a time; warp w
+// takes groups w, w + kDeleteWarps, ... All of a group's removals of the chunk
+// and the list's last entries are read at once, one per lane; the swap-removes
+// then run in order over the warp's registers, and each surviving move is
+// stored once. The lists are those of one removal after another.
+static __device__ __noinline__ void apply_delete_block(const StoreView& S, uint32_t u, const uint32_t* seg_slot,
+                                                       uint32_t len, AliasScratch& A, BlockDelete& B) {
+  const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+  VertexMeta M = S.meta[u];
+  GroupDesc G = S.gdesc[(size_t)u * kBits + lane];
+  VertexRec R = S.vrec[u];
+  const uint32_t cnt0 = G.cnt, cap0 = group_cap(G);
+  uint32_t* const bpv = S.bp + M.bpoff;
+  uint32_t cnt = cnt0, rejected = 0;  // cnt: of the groups this warp takes
+  for (uint32_t c = 0; c < len; c += 32) {
+    const uint32_t i = c + lane;
+    uint32_t slot = 0xffffffffu;
+    EdgeRec e{0, 0, 0, 0};
+    bool valid = false;
+    if (wi == 0) {
+      if (i < len) slot = seg_slot[i];
+      if (i < len && slot < M.ecnt) e = S.edges[M.eoff + slot];
+      const bool dup = (__match_any_sync(kFull, slot) & lanemask_lt()) != 0;
+      valid = i < len && e.w != 0 && !dup;
+      M.live -= __popc(__ballot_sync(kFull, valid));
+      rejected += __popc(__ballot_sync(kFull, i < len && !valid));
+      B.w[lane] = valid ? e.w : 0u;
+      B.ebp[lane] = e.ebp;
+    }
+    __syncthreads();
+    const uint32_t wd = B.w[lane], run = B.ebp[lane];
+    for (int k = wi; k < kBits; k += kDeleteWarps) {
+      const bool has = (wd >> k) & 1u;
+      const uint32_t mask = __ballot_sync(kFull, has);
+      const int r = __popc(mask);
+      if (!r) continue;
+      if (has) B.order[wi][__popc(mask & lanemask_lt())] = run + __popc(wd & ((1u << k) - 1u));
+      __syncwarp();
+      const uint32_t c0 = __shfl_sync(kFull, cnt, k);
+      const size_t gb = (size_t)__shfl_sync(kFull, group_base(G), k) * 4;
+      // Lane t < r: removal t, and the entry at the list's position c0 - 1 - t.
+      uint32_t bpi = 0xffffffffu, pos = 0, tv = 0, tbi = 0xffffffffu;
+      if (lane < r) {
+        bpi = B.order[wi][lane];
+        pos = bpv[bpi];
+        tbi = S.gs[gb + c0 - 1 - lane];
+        tv = S.gv[gb + c0 - 1 - lane];
+      }
+      uint32_t to = 0xffffffffu, mv = 0, mbi = 0;  // lane t: the move removal t makes, while it stands
+      for (int t = 0; t < r; ++t) {
+        const uint32_t p = __shfl_sync(kFull, pos, t), v = __shfl_sync(kFull, tv, t), b = __shfl_sync(kFull, tbi, t);
+        if (p == c0 - 1 - t) continue;  // the last entry itself
+        if (lane > t && p == c0 - 1 - lane) tv = v, tbi = b;  // a later last entry
+        if (lane > t && bpi == b) pos = p;                    // a later removal moved
+        if (lane < t && to == p) to = 0xffffffffu;            // an earlier move's entry is gone
+        if (lane == t) to = p, mv = v, mbi = b;
+      }
+      // Moves into positions past the new end moved on, or went.
+      if (to < c0 - r) {
+        S.gv[gb + to] = mv;
+        S.gs[gb + to] = mbi;
+        bpv[mbi] = to;
+      }
+      if (lane == k) cnt = c0 - r;
+      __syncwarp();  // the order entries are reused
+    }
+    if (valid) {
+      S.edges[M.eoff + slot].w = 0u;
+      if (S.node2vec && R.hmask) hash_sub(S.hash + R.hoff, R.hmask, e.v, e.w);
+    }
+    __syncthreads();
+  }
+  if (lane % kDeleteWarps == wi) B.cnt[lane] = cnt;
+  __syncthreads();
+  if (wi == 0) {
+    if (rejected && lane == 0) {
+      atomicAdd(&S.err[1], rejected);
+      set_err(S.err, E_INVALID_SLOT);
+    }
+    cnt = B.cnt[lane];
+    const size_t gb = (size_t)group_base(G) * 4;
+    R.m = warp_build_alias(lane, cnt, group_base(G), cnt == 1 ? S.gv[gb] : 0u, S.alias + R.aoff, &A);
+    if (cnt != cnt0) {
+      G.cnt = cnt;
+      G.roomy = group_roomy(cnt, cap0);
+      S.gdesc[(size_t)u * kBits + lane] = G;
+    }
+    if (lane == 0) {
+      S.meta[u] = M;
+      S.vrec[u] = R;
+    }
+  }
+  __syncthreads();  // B is reused by the block's next segment
 }
 
 }  // namespace bingo
