@@ -546,9 +546,11 @@ __global__ void __launch_bounds__(kBlock) k_pair_slots(StoreView S, const unsign
 static_assert(kBlock % 32 == 0, "whole warps");
 
 // Resident 256-thread blocks per SM each walk variant is compiled for
-// (register budget 65536 / (256 * blocks)).
-constexpr int walk_min_blocks(int app, bool multi) {
-  return app == APP_SAMPLING ? 8 : app == APP_DEEPWALK ? 5 : app == APP_PPR ? 5 : 4;
+// (register budget 65536 / (256 * blocks)). node2vec, bound by DRAM, runs best
+// at 4 (1 M walks: 1953 us; 2209 at 3); mixed tables, where the longest walks'
+// steps set the time, at 3 (16 jobs: 1716 us; 1833 at 4, 1929 at 2).
+constexpr int walk_min_blocks(int app) {
+  return app == APP_SAMPLING ? 8 : app == APP_DEEPWALK || app == APP_PPR ? 5 : app == APP_NODE2VEC ? 4 : 3;
 }
 // Entries of a lane's output line (RowStage): 128 bytes, and 64 where the
 // trial scratch also takes shared memory (L1 holds the reads in flight, so
@@ -569,7 +571,7 @@ __device__ __forceinline__ uint32_t job_of_item(const uint32_t* __restrict__ pre
 }
 
 template <int APP, bool MULTI>
-__global__ void __launch_bounds__(kBlock, walk_min_blocks(APP, MULTI))
+__global__ void __launch_bounds__(kBlock, walk_min_blocks(APP))
     k_walk(WalkView W, WalkJobDev J0, const WalkJobDev* __restrict__ jobs, const uint32_t* __restrict__ prefix,
            uint32_t n_jobs, uint32_t total, uint32_t* queue, uint32_t chunk) {
   constexpr int kLine = walk_line(APP);
@@ -766,7 +768,7 @@ void walk_carveouts(int device) {
   if (std::find(done.begin(), done.end(), device) != done.end()) return;
   walk_carveout<APP_DEEPWALK, false>(4), walk_carveout<APP_DEEPWALK, true>(4);
   walk_carveout<APP_PPR, false>(4), walk_carveout<APP_PPR, true>(4);
-  walk_carveout<APP_NODE2VEC, false>(4), walk_carveout<APP_NODE2VEC, true>(4), walk_carveout<-1, true>(4);
+  walk_carveout<APP_NODE2VEC, false>(4), walk_carveout<APP_NODE2VEC, true>(4), walk_carveout<-1, true>(3);
   done.push_back(device);
 }
 
@@ -1553,7 +1555,8 @@ void Engine::load_f32(const uint32_t* src, const uint32_t* dst, const float* w, 
   if (m >= (1ull << 31)) throw Error(BINGO_ERR_UNSUPPORTED, "more than 2^31 edges in one load");
   const uint32_t* q = m ? fixed_weights(w, m) : nullptr;
   load(src, dst, m ? q : nullptr, m, n);
-  fw_in_.release(), fw_fixed_.release();
+  // Kept for the next load like the scratch slab, while small.
+  if (fw_in_.bytes + fw_fixed_.bytes > std::max<size_t>(load_slab_.bytes / 4, 64u << 20)) fw_in_.release(), fw_fixed_.release();
 }
 
 void Engine::insert_f32(const uint32_t* src, const uint32_t* dst, const float* w, uint64_t k, uint32_t* out_slots) {

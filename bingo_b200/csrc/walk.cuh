@@ -266,6 +266,31 @@ struct TrialScratch {
   uint16_t item[kTrialItems];  // lane | trial << 8 | node2vec trial << 15
 };
 
+// One draw: trial t of step j of walk i at a vertex with m alias slots from
+// aoff; `second`: a node2vec trial, with acceptance draw ax against the
+// previous vertex and its adjacency index.
+struct Trial {
+  int32_t x;
+  bool ok, probe;  // accepted; looked up the adjacency index
+};
+__device__ __forceinline__ Trial draw_trial(const WalkView& W, const WalkJobDev& V, uint32_t i, uint32_t j, uint32_t t,
+                                            uint32_t aoff, uint32_t m, bool second, unsigned long long ax,
+                                            int32_t prev, uint32_t phoff, uint32_t phmask) {
+  Trial r{(int32_t)sample_at(W, aoff, m, philox(i, j, 2 * t, V.job, V.k0, V.k1)), true, false};
+  if (second) {
+    // Accepted with probability weight(class(x)) / envelope; the adjacency
+    // index is read only where the class decides.
+    if (r.x == prev) {
+      r.ok = ax < V.thr_ret;
+    } else if (ax >= (V.thr_in < V.thr_out ? V.thr_in : V.thr_out)) {
+      r.probe = true;
+      r.ok = ax < (hash_has(W.hash + phoff, phmask, (uint32_t)r.x) ? V.thr_in : V.thr_out);
+    }
+    r.ok = r.ok || t + 1 == kMaxNode2vecTrials;
+  }
+  return r;
+}
+
 // One step of every active lane's walk; `jobs` is the job table (jid indexes
 // it) or the one job.
 template <int APP>
@@ -304,53 +329,55 @@ __device__ __forceinline__ Proposal warp_propose(const WalkView& W, const WalkJo
   const bool ret = n2v && R.m && s.t == 0 && J.ret_excess > 0.0;
   HashPeek rp;
   if (ret) hash_peek(rp, W.hash + R.hoff, R.hmask, (uint32_t)s.prev);
-  const uint32_t incl = warp_incl_scan(n, lane), off = incl - n;
-  const uint32_t total = __shfl_sync(kFull, incl, 31);
-  for (uint32_t k = 0; k < n; ++k) sc.item[off + k] = (uint16_t)(lane | k << 8 | (n2v ? 1u << 15 : 0u));
-  __syncwarp();
   constexpr uint32_t kNone = 0xffffffffu;
   uint32_t won = kNone, probed = 0;  // the accepted trial; this lane's trials that looked up the adjacency index
-  for (uint32_t base = 0; base < total; base += 32) {
-    const bool valid = base + lane < total;
-    const uint32_t it = valid ? sc.item[base + lane] : 0u;
-    const int src = it & 31;
-    const uint32_t vi = __shfl_sync(kFull, s.i, src), vj = __shfl_sync(kFull, s.j, src);
-    const uint32_t vt = __shfl_sync(kFull, s.t, src) + ((it >> 8) & 0x7f);
-    const uint32_t vaoff = __shfl_sync(kFull, R.aoff, src), vm = __shfl_sync(kFull, R.m, src);
-    const int32_t vprev = __shfl_sync(kFull, s.prev, src);
-    const uint32_t vphoff = __shfl_sync(kFull, s.phoff, src), vphmask = __shfl_sync(kFull, s.phmask, src);
-    const WalkJobDev& V = jobs[__shfl_sync(kFull, jid, src)];
-    int32_t x = -1;
-    bool ok = valid, probe = false;
-    if (valid) x = (int32_t)sample_at(W, vaoff, vm, philox(vi, vj, 2 * vt, V.job, V.k0, V.k1));
-    if (it >> 15) {
-      // Accepted with probability weight(class(x)) / envelope; the adjacency
-      // index is read only where the class decides.
-      const unsigned long long ax = sc.ax[__popc(am & ((1u << src) - 1u)) * cap + ((it >> 8) & 0x7f)];
-      if (x == vprev) {
-        ok = ax < V.thr_ret;
-      } else if (ax >= (V.thr_in < V.thr_out ? V.thr_in : V.thr_out)) {
-        probe = true;
-        ok = ax < (hash_has(W.hash + vphoff, vphmask, (uint32_t)x) ? V.thr_in : V.thr_out);
-      }
-      ok = ok || vt + 1 == kMaxNode2vecTrials;
+  if (APP < 0 && !__any_sync(kFull, n > 1)) {
+    // A draw per lane at most (DeepWalk, PPR, q <= 1), as in many warps of a
+    // mixed table: each draws its own. (A table of node2vec alone seldom gets
+    // here: 1952 us without, 1958 with.)
+    if (n) {
+      const Trial r = draw_trial(W, J, s.i, s.j, s.t, R.aoff, R.m, n2v, n2v ? sc.ax[mine] : 0u, s.prev, s.phoff, s.phmask);
+      if (r.ok) won = 0, p.x = r.x;
+      probed = r.probe;
     }
-    const uint32_t oks = __ballot_sync(kFull, ok), probes = __ballot_sync(kFull, probe);
-    const uint32_t lo = max(off, base), hi = min(off + n, base + 32);
-    int from = 0;
-    bool take = false;
-    if (lo < hi && won == kNone) {  // this lane's trials among the 32
-      const uint32_t here = kFull >> (32 - (hi - lo)), first = lo - base;
-      const uint32_t acc = (oks >> first) & here;
-      probed |= ((probes >> first) & here) << (lo - off);
-      if (acc) {
-        from = (int)(first + __ffs(acc) - 1);
-        won = base + from - off;
-        take = true;
+  } else {
+    const uint32_t incl = warp_incl_scan(n, lane), off = incl - n;
+    const uint32_t total = __shfl_sync(kFull, incl, 31);
+    for (uint32_t k = 0; k < n; ++k) sc.item[off + k] = (uint16_t)(lane | k << 8 | (n2v ? 1u << 15 : 0u));
+    __syncwarp();
+    for (uint32_t base = 0; base < total; base += 32) {
+      const bool valid = base + lane < total;
+      const uint32_t it = valid ? sc.item[base + lane] : 0u;
+      const int src = it & 31;
+      const uint32_t k = (it >> 8) & 0x7f;
+      const uint32_t vi = __shfl_sync(kFull, s.i, src), vj = __shfl_sync(kFull, s.j, src);
+      const uint32_t vt = __shfl_sync(kFull, s.t, src) + k;
+      const uint32_t vaoff = __shfl_sync(kFull, R.aoff, src), vm = __shfl_sync(kFull, R.m, src);
+      const int32_t vprev = __shfl_sync(kFull, s.prev, src);
+      const uint32_t vphoff = __shfl_sync(kFull, s.phoff, src), vphmask = __shfl_sync(kFull, s.phmask, src);
+      const WalkJobDev& V = jobs[__shfl_sync(kFull, jid, src)];
+      Trial r{-1, false, false};
+      if (valid) {
+        const uint32_t ax = sc.ax[__popc(am & ((1u << src) - 1u)) * cap + k];
+        r = draw_trial(W, V, vi, vj, vt, vaoff, vm, it >> 15, ax, vprev, vphoff, vphmask);
       }
+      const uint32_t oks = __ballot_sync(kFull, r.ok), probes = __ballot_sync(kFull, r.probe);
+      const uint32_t lo = max(off, base), hi = min(off + n, base + 32);
+      int from = 0;
+      bool take = false;
+      if (lo < hi && won == kNone) {  // this lane's trials among the 32
+        const uint32_t here = kFull >> (32 - (hi - lo)), first = lo - base;
+        const uint32_t acc = (oks >> first) & here;
+        probed |= ((probes >> first) & here) << (lo - off);
+        if (acc) {
+          from = (int)(first + __ffs(acc) - 1);
+          won = base + from - off;
+          take = true;
+        }
+      }
+      const int32_t x = __shfl_sync(kFull, r.x, from);
+      if (take) p.x = x;
     }
-    x = __shfl_sync(kFull, x, from);
-    if (take) p.x = x;
   }
   if (n2v && R.m) {
     // Return region: when 1/p exceeds the envelope max(1, 1/q), the excess
