@@ -345,10 +345,15 @@ __device__ __forceinline__ uint32_t segs_per_warp(uint32_t nS, uint32_t warps) {
   return min(8u, max(1u, nS / warps));
 }
 
-__global__ void __launch_bounds__(kBlock, 4) k_apply_insert(const __grid_constant__ StoreView S, const uint32_t* skey, const uint32_t* sv,
+// LOAD: a whole graph's edges, whose back-pointers are staged (append_range);
+// a streaming batch keeps its shared memory small instead, so that the next
+// batch's grouping cluster can start beside it.
+template <bool LOAD>
+__global__ void __launch_bounds__(kBlock, 4) k_apply_insert(const __grid_constant__ StoreView S,
+                                                         const uint32_t* skey, const uint32_t* sv,
                                                          const uint32_t* sw, const uint32_t* sorig,
                                                          const uint32_t* seg, const uint32_t* nseg,
-                                                         unsigned long long k, uint32_t ks, const uint32_t* ctl,
+                                                         unsigned long long k, uint32_t ks, uint32_t* ctl,
                                                          const ArenaNeed* excl, const unsigned long long* boff,
                                                          const unsigned long long* base,
                                                          const __grid_constant__ HostReserve hr,
@@ -358,6 +363,8 @@ __global__ void __launch_bounds__(kBlock, 4) k_apply_insert(const __grid_constan
   pdl_trigger();
   __shared__ AliasScratch asc[kBlock / 32];
   __shared__ BlockAppend ba;
+  __shared__ uint32_t bps[LOAD ? kBlock / 32 : 1][LOAD ? kStageEntries : 1], ticket;
+  uint32_t* const stage = LOAD ? bps[threadIdx.x / 32] : nullptr;
   if (*ctl) return;
   if (!base && blockIdx.x == 0) {
 #pragma unroll
@@ -365,7 +372,19 @@ __global__ void __launch_bounds__(kBlock, 4) k_apply_insert(const __grid_constan
       if (threadIdx.x == a) S.top[a] = hr.top[a];  // constant indices keep hr in parameter space
   }
   const uint32_t nS = *nseg, nb = plan_blocks(ks), nbig = ctl[1];
-  for (uint32_t q = blockIdx.x; q < nbig; q += gridDim.x) {
+  for (uint32_t turn = 0;; ++turn) {
+    // Listed segments differ in length by orders of magnitude: many are taken
+    // in turn by whichever block is free (ctl[3]).
+    uint32_t q = blockIdx.x;
+    if (nbig > gridDim.x) {
+      if (threadIdx.x == 0) ticket = atomicAdd(ctl + 3, 1u);
+      __syncthreads();
+      q = ticket;
+      __syncthreads();
+    } else if (turn) {
+      break;
+    }
+    if (q >= nbig) break;
     const uint32_t s = big[q];
     uint32_t b, e;
     seg_bounds(seg, nS, s, k, &b, &e);
@@ -373,17 +392,26 @@ __global__ void __launch_bounds__(kBlock, 4) k_apply_insert(const __grid_constan
 #pragma unroll
     for (int a = 0; a < kArenas; ++a)
       res.v[a] = (base ? base[a] : hr.base[a]) + boff[(size_t)a * nb + s / kPlanSegs] + (excl[s].v[a] & ~kBigFlag);
-    apply_append_block(S, skey[b], sv + b, sw + b, sorig + b, e - b, out_slots, res, asc[threadIdx.x / 32], ba);
+    apply_append_block(S, skey[b], sv + b, sw + b, sorig + b, e - b, out_slots, res, asc[threadIdx.x / 32], ba,
+                       stage);
   }
-  // The other segments, one warp each, `per` consecutive ones at a time;
-  // blocks that had a listed one leave them to the rest while those are the
-  // most.
-  const uint32_t skip = nbig < gridDim.x / 2 ? nbig : 0u;
+  // The other segments, one warp each, `per` consecutive ones at a time: in
+  // turn by whichever warp is free when there are many (ctl[2]), else dealt
+  // out; blocks that had a listed one then leave them to the rest while those
+  // are the most.
+  const bool many = nS > 16u * gridDim.x * (kBlock / 32);
+  const uint32_t skip = !many && nbig < gridDim.x / 2 ? nbig : 0u;
   if (blockIdx.x < skip) return;
   const int lane = threadIdx.x & 31;
   AliasScratch& A = asc[threadIdx.x / 32];
   const uint32_t warps = (gridDim.x - skip) * (kBlock / 32), per = segs_per_warp(nS, warps);
-  for (uint32_t s0 = ((blockIdx.x - skip) * kBlock + threadIdx.x) / 32 * per; s0 < nS; s0 += warps * per) {
+  uint32_t s0 = ((blockIdx.x - skip) * kBlock + threadIdx.x) / 32 * per;
+  for (;; s0 += warps * per) {
+    if (many) {
+      if (lane == 0) s0 = atomicAdd(ctl + 2, per);
+      s0 = __shfl_sync(kFull, s0, 0);
+    }
+    if (s0 >= nS) break;
     // Lane i: segment s0 + i.
     const uint32_t s = s0 + lane;
     uint32_t b = 0, e = 0, u = 0xffffffffu;
@@ -398,7 +426,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_apply_insert(const __grid_constan
       auto res = [&](int a) {
         return (base ? base[a] : hr.base[a]) + boff[(size_t)a * nb + vs / kPlanSegs] + (excl[vs].v[a] & ~kBigFlag);
       };
-      apply_append(S, __shfl_sync(kFull, u, src), sv + vb, sw + vb, sorig + vb, ve - vb, out_slots, res, A);
+      apply_append(S, __shfl_sync(kFull, u, src), sv + vb, sw + vb, sorig + vb, ve - vb, out_slots, res, A, stage);
     }
   }
 }
@@ -1338,8 +1366,8 @@ void Engine::run_insert(uint64_t k, uint32_t* dev_out_slots, bool load_mode, uin
   h_plan_[kPlanStatusSlot] = 0;  // k_totals publishes the plan and then a nonzero status here
   plan_needs(S0, k, ks, d_plan_, load_mode ? kReserveNone : kReservePublish);
   auto apply = [&](const StoreView& S, const unsigned long long* dev_base, const HostReserve& hr) {
-    launch_pdl(k_apply_insert, grid_for((unsigned long long)ks * 32, kBlock, tuning_.apply_blocks_per_sm), kBlock,
-               stream_, S, key_s_.as<uint32_t>(), sa_.as<uint32_t>(), sb_.as<uint32_t>(), perm_.as<uint32_t>(),
+    launch_pdl(load_mode ? k_apply_insert<true> : k_apply_insert<false>,
+               grid_for((unsigned long long)ks * 32, kBlock, tuning_.apply_blocks_per_sm), kBlock, stream_, S, key_s_.as<uint32_t>(), sa_.as<uint32_t>(), sb_.as<uint32_t>(), perm_.as<uint32_t>(),
                seg_.as<uint32_t>(), nseg_.as<uint32_t>(), k, ks, ctl_.as<uint32_t>(), scan_.as<ArenaNeed>(),
                need_.as<unsigned long long>(), dev_base, hr, big_.as<uint32_t>(), dev_out_slots);
     cuda_check(cudaGetLastError(), "apply insert");
@@ -1904,7 +1932,7 @@ void Engine::enqueue_insert(const uint32_t* a, const uint32_t* b, const uint32_t
   group_by_vertex(a, b, c, k, true);
   const StoreView S = view();
   plan_needs(S, k, ks, nullptr, kReserveSticky);
-  launch_pdl(k_apply_insert, grid_for((unsigned long long)ks * 32, kBlock, tuning_.apply_blocks_per_sm), kBlock,
+  launch_pdl(k_apply_insert<false>, grid_for((unsigned long long)ks * 32, kBlock, tuning_.apply_blocks_per_sm), kBlock,
              stream_, S, key_s_.as<uint32_t>(), sa_.as<uint32_t>(), sb_.as<uint32_t>(), perm_.as<uint32_t>(),
              seg_.as<uint32_t>(), nseg_.as<uint32_t>(), k, ks, ctl_.as<uint32_t>(), scan_.as<ArenaNeed>(),
              need_.as<unsigned long long>(), base_.as<unsigned long long>(), HostReserve{}, big_.as<uint32_t>(), out_slots);

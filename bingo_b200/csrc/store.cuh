@@ -278,11 +278,17 @@ __device__ __forceinline__ void warp_copy_u32(uint32_t* dst, const uint32_t* src
 // Appends edges [from, to) of a segment in batch order (one warp): M with the
 // vertex's arrays and its slot count before the segment; G.cnt and bpbase are
 // the positions this range starts at and end past it. `single` becomes the
-// first member of a group that was empty.
+// first member of a group that was empty and gets one.
+//
+// stage (kStageEntries words of shared memory, or null): the 32 edges' back-
+// pointers are collected there and written together. Written bit by bit, each
+// of an edge's back-pointers is a store of its own to the same sector: two
+// thirds of a load's writes to L2.
+constexpr uint32_t kStageEntries = 512;
 __device__ __forceinline__ void append_range(const StoreView& S, const VertexMeta& M, GroupDesc& G, uint32_t& bpbase,
                                              uint32_t& single, const uint32_t* seg_v, const uint32_t* seg_w,
                                              const uint32_t* seg_orig, uint32_t from, uint32_t to,
-                                             uint32_t* out_slots) {
+                                             uint32_t* out_slots, uint32_t* stage) {
   const int lane = threadIdx.x & 31;
   for (uint32_t c = from; c < to; c += 32) {
     const uint32_t i = c + lane;
@@ -290,13 +296,14 @@ __device__ __forceinline__ void append_range(const StoreView& S, const VertexMet
     const uint32_t v = valid ? seg_v[i] : 0u, w = valid ? seg_w[i] : 0u;
     const uint32_t pc = __popc(w);
     const uint32_t incl = warp_incl_scan(pc, lane);
-    const uint32_t ebp = bpbase + incl - pc;
-    bpbase += __shfl_sync(kFull, incl, 31);
+    const uint32_t total = __shfl_sync(kFull, incl, 31);
     const uint32_t slot = M.ecnt + i;
+    uint32_t bi = bpbase + incl - pc;  // this edge's next back-pointer
     if (valid) {
-      S.edges[M.eoff + slot] = EdgeRec{v, w, ebp, 0u};
+      S.edges[M.eoff + slot] = EdgeRec{v, w, bi, 0u};
       if (out_slots) out_slots[seg_orig[i]] = slot;
     }
+    const bool staged = stage && total <= kStageEntries;
     uint32_t present = __reduce_or_sync(kFull, w);
     while (present) {
       const int k = __ffs(present) - 1;
@@ -305,18 +312,29 @@ __device__ __forceinline__ void append_range(const StoreView& S, const VertexMet
       const uint32_t b = __ballot_sync(kFull, has);
       const uint32_t kcnt = __shfl_sync(kFull, G.cnt, k), kbase = __shfl_sync(kFull, group_base(G), k);
       if (has) {
-        const uint32_t pos = kcnt + __popc(b & lanemask_lt()), bi = ebp + __popc(w & ((1u << k) - 1u));
+        const uint32_t pos = kcnt + __popc(b & lanemask_lt());
         const size_t e = (size_t)kbase * 4 + pos;
         S.gv[e] = v;
         S.gs[e] = bi;
-        S.bp[M.bpoff + bi] = pos;
+        if (staged)
+          stage[bi - bpbase] = pos;
+        else
+          S.bp[M.bpoff + bi] = pos;
+        ++bi;
       }
-      const uint32_t first_v = __shfl_sync(kFull, v, __ffs(b) - 1);  // b != 0: bit k is present
-      if (lane == k) {
-        if (kcnt == 0) single = first_v;
-        G.cnt += __popc(b);
+      if (kcnt == 0) {  // b != 0: bit k is present
+        const uint32_t first_v = __shfl_sync(kFull, v, __ffs(b) - 1);
+        if (lane == k) single = first_v;
       }
+      if (lane == k) G.cnt += __popc(b);
     }
+    if (staged) {
+      __syncwarp();
+      uint32_t* const out = S.bp + M.bpoff + bpbase;
+      for (uint32_t t = lane; t < total; t += 32) out[t] = stage[t];
+      __syncwarp();
+    }
+    bpbase += total;
   }
 }
 
@@ -335,7 +353,7 @@ constexpr unsigned long long kBigFlag = 1ull << 63;  // marks such a segment in 
 // ---------------------------------------------------------------------------
 // Apply a growth plan (relocations drawn from per-arena bases reserved for
 // this segment), append the segment's edges in order, refresh the adjacency
-// index and stage the alias table (alias_finish writes it). Replaces NodeData::copy / insert /
+// index and rebuild the alias table. Replaces NodeData::copy / insert /
 // buildAliasTable (include/Bingo.cuh:95-110, :182-198, :111-158) and the host
 // reMalloc round trip (include/operation.cuh:163-174).
 //
@@ -345,7 +363,7 @@ constexpr unsigned long long kBigFlag = 1ull << 63;  // marks such a segment in 
 template <class Reserved>
 static __device__ __forceinline__ void apply_append(const StoreView& S, uint32_t u, const uint32_t* seg_v, const uint32_t* seg_w,
                              const uint32_t* seg_orig, uint32_t len, uint32_t* out_slots,
-                             const Reserved& res, AliasScratch& B) {
+                             const Reserved& res, AliasScratch& B, uint32_t* stage) {
   const int lane = threadIdx.x & 31;
   VertexMeta M = S.meta[u];
   GroupDesc G = S.gdesc[(size_t)u * kBits + lane];
@@ -433,7 +451,7 @@ static __device__ __forceinline__ void apply_append(const StoreView& S, uint32_t
     }
     bpbase += __popc(w);
   } else {
-    append_range(S, M, G, bpbase, single, seg_v, seg_w, seg_orig, 0, len, out_slots);
+    append_range(S, M, G, bpbase, single, seg_v, seg_w, seg_orig, 0, len, out_slots, stage);
   }
   M.ecnt += len;
   M.bpcnt = bpbase;
@@ -505,7 +523,7 @@ struct BlockAppend {
 static __device__ __noinline__ void apply_append_block(const StoreView& S, uint32_t u, const uint32_t* seg_v,
                                                        const uint32_t* seg_w, const uint32_t* seg_orig, uint32_t len,
                                                        uint32_t* out_slots, ArenaNeed at, AliasScratch& A,
-                                                       BlockAppend& B) {
+                                                       BlockAppend& B, uint32_t* stage) {
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
   VertexMeta M = S.meta[u];
   GroupDesc G = S.gdesc[(size_t)u * kBits + lane];
@@ -577,7 +595,7 @@ static __device__ __noinline__ void apply_append_block(const StoreView& S, uint3
   // --- append ---
   G.cnt += before;
   uint32_t bpbase = M.bpcnt + pc_before, single = 0xffffffffu;
-  append_range(S, M, G, bpbase, single, seg_v, seg_w, seg_orig, from, to, out_slots);
+  append_range(S, M, G, bpbase, single, seg_v, seg_w, seg_orig, from, to, out_slots, stage);
   if (cnt0 == 0 && before == 0 && add) B.single[lane] = single;  // this range holds the group's first member
   M.ecnt += len;
   M.bpcnt += pc_total;
