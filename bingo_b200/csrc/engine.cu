@@ -578,7 +578,7 @@ static_assert(kBlock % 32 == 0, "whole warps");
 // at 4 (1 M walks: 1953 us; 2209 at 3); mixed tables, where the longest walks'
 // steps set the time, at 3 (16 jobs: 1716 us; 1833 at 4, 1929 at 2).
 constexpr int walk_min_blocks(int app) {
-  return app == APP_SAMPLING ? 8 : app == APP_DEEPWALK || app == APP_PPR ? 5 : app == APP_NODE2VEC ? 4 : 3;
+  return app == APP_SAMPLING ? 8 : app < 0 ? 3 : 4;
 }
 // Entries of a lane's output line (RowStage): 128 bytes, and 64 where the
 // trial scratch also takes shared memory (L1 holds the reads in flight, so
@@ -620,6 +620,9 @@ __global__ void __launch_bounds__(kBlock, walk_min_blocks(APP))
   uint32_t jid = 0, moves = 0, wb = 0, we = 0;
   s.trials = 0, s.probes = 0;
   s.i = s.j = s.cur = s.lo = s.phoff = s.phmask = s.t = 0, s.row = nullptr, s.prev = -1, s.region = 0;
+  s.R = VertexRec{0, 0, 0, 0};
+  Rand4 ahead{0, 0, 0, 0};
+  constexpr int A = APP == APP_SAMPLING ? APP_DEEPWALK : APP;
   bool active = false, drained = false;
   const uint32_t warps = gridDim.x * (kBlock / 32);
   // A small launch's walks spread over all its warps (walks that take trials
@@ -647,10 +650,14 @@ __global__ void __launch_bounds__(kBlock, walk_min_blocks(APP))
       if (!active && rank < take) {
         const uint32_t item = wb + rank;
         if (!MULTI) {
-          active = walk_begin<APP, kLine>(W, J0, item, s, buf, moves);
+          active = walk_begin<APP, kLine, !kTrials>(W, J0, item, s, buf, moves);
         } else {
           jid = job_of_item(prefix, n_jobs, item);
-          active = walk_begin<APP, kLine>(W, jobs[jid], item - prefix[jid], s, buf, moves);
+          active = walk_begin<APP, kLine, !kTrials>(W, jobs[jid], item - prefix[jid], s, buf, moves);
+        }
+        if (A == APP_DEEPWALK && active) {
+          const WalkJobDev& J = MULTI ? jobs[jid] : J0;
+          ahead = philox(s.i, 1, 0, J.job, J.k0, J.k1);
         }
       }
       wb += take;
@@ -661,7 +668,6 @@ __global__ void __launch_bounds__(kBlock, walk_min_blocks(APP))
       continue;
     }
     if (!kRows) continue;
-    constexpr int A = APP == APP_SAMPLING ? APP_DEEPWALK : APP;
     const WalkJobDev& J = MULTI ? jobs[jid] : J0;
     bool out = false, end = false;
     uint32_t pos = 0;
@@ -669,9 +675,9 @@ __global__ void __launch_bounds__(kBlock, walk_min_blocks(APP))
     if (kTrials)
       p = warp_propose<A>(W, MULTI ? jobs : &one, jid, s, active, trials[threadIdx.x / 32]);
     else if (active)
-      p = walk_propose<A>(W, J, s);
+      p = walk_propose<A>(W, J, s, ahead);
     if (active && p.ok) {
-      active = walk_commit<A, kLine>(J, s, p, buf, moves, out, pos);
+      active = walk_commit<A, kLine, !kTrials>(W, J, s, p, buf, moves, out, pos);
       end = !active;
     }
     Stage::flush(wbuf, out, end, s, pos, J.L);

@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(kServeBlock, 4)
     uint32_t pos = 0;
     const Proposal p = warp_propose<-1>(W, wjc, (uint32_t)lane, s, active, trials[threadIdx.x / 32]);
     if (active && p.ok) {
-      active = walk_commit<-1, kServeLine>(J, s, p, wbuf + mine, moves, out, pos);
+      active = walk_commit<-1, kServeLine>(W, J, s, p, wbuf + mine, moves, out, pos);
       end = !active;
     }
     Stage::flush(wbuf, out, end, s, pos, out ? J.L : 0u);

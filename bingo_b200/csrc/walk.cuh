@@ -113,6 +113,7 @@ struct LaneWalk {
   uint32_t i;      // walk index within its job
   uint32_t j;      // step being produced
   uint32_t cur;    // current vertex
+  VertexRec R;     // first-order kernels: its record, requested as soon as the vertex is known
   uint32_t lo;     // first entry of the open output line that belongs to this row
   int32_t* row;    // the walk's output row
   int32_t prev;    // previous vertex (node2vec), -1 before the first move
@@ -173,7 +174,7 @@ struct RowStage {
 
 // Starts walk i; returns true if it still has steps to produce. Sampling jobs
 // and rows of one position complete here. `buf`: this lane's line entries.
-template <int APP, int LINE>
+template <int APP, int LINE, bool AHEAD = false>
 __device__ __forceinline__ bool walk_begin(const WalkView& W, const WalkJobDev& J, uint32_t i, LaneWalk& s,
                                            int32_t* buf, uint32_t& moves) {
   const uint32_t start = J.starts ? J.starts[i] : J.first + i;
@@ -214,6 +215,7 @@ __device__ __forceinline__ bool walk_begin(const WalkView& W, const WalkJobDev& 
   s.i = i;
   s.j = 1;
   s.cur = start;
+  if (AHEAD) s.R = load_vrec(W, start);
   s.prev = -1;
   s.t = 0;
   return true;
@@ -227,19 +229,30 @@ struct Proposal {
   uint32_t hoff, hmask;  // the current vertex's adjacency index (node2vec)
 };
 
-// Draws the next vertex of a first-order walk (DeepWalk, PPR). The Philox
-// blocks depend on no load: they are drawn while the vertex record is on its
-// way (R-MAT 14, 16,384 walks x 80: 85 -> 79 us).
+// Draws the next vertex of a first-order walk (DeepWalk, PPR). A small launch
+// is bound by the chain of a step's three reads and what lies between them, so
+// little else does: the next vertex's record is requested (walk_commit) before
+// the row is written and new walks are started, and the Philox blocks, which
+// depend on no read, are drawn under one. DeepWalk draws `ahead`, step j + 1's
+// under step j's member read (R-MAT 14, 16,384 walks x 80: 85 us with the draws
+// after the record's read, 72 under it, 68 so); PPR's two blocks are longer
+// than that read and stay under the record's (100,003 walks: 225 us, 227
+// ahead).
 template <int APP>
-__device__ __forceinline__ Proposal walk_propose(const WalkView& W, const WalkJobDev& J, const LaneWalk& s) {
-  const VertexRec R = load_vrec(W, s.cur);
-  Rand4 r = philox(s.i, s.j, 0, J.job, J.k0, J.k1);
-  uint32_t ax = 0;
-  if (APP == APP_PPR) ax = philox(s.i, s.j, 1, J.job, J.k0, J.k1).x;
-  asm volatile("" : "+r"(r.x), "+r"(r.y), "+r"(r.z), "+r"(r.w), "+r"(ax));  // drawn before R is looked at
+__device__ __forceinline__ Proposal walk_propose(const WalkView& W, const WalkJobDev& J, const LaneWalk& s,
+                                                 Rand4& ahead) {
   Proposal p{-1, true, false, 0, 0};
-  if (APP == APP_PPR) p.stop = (unsigned long long)ax < J.thr_stop;
-  if (R.m) p.x = (int32_t)sample_at(W, R.aoff, R.m, r);
+  if (APP == APP_PPR) {
+    Rand4 r = philox(s.i, s.j, 0, J.job, J.k0, J.k1);
+    uint32_t ax = philox(s.i, s.j, 1, J.job, J.k0, J.k1).x;
+    asm volatile("" : "+r"(r.x), "+r"(r.y), "+r"(r.z), "+r"(r.w), "+r"(ax));  // drawn before R is looked at
+    p.stop = (unsigned long long)ax < J.thr_stop;
+    if (s.R.m) p.x = (int32_t)sample_at(W, s.R.aoff, s.R.m, r);
+  } else {
+    if (s.R.m) p.x = (int32_t)sample_at(W, s.R.aoff, s.R.m, ahead);
+    ahead = philox(s.i, s.j + 1, 0, J.job, J.k0, J.k1);
+    asm volatile("" : "+r"(p.x), "+r"(ahead.x), "+r"(ahead.y), "+r"(ahead.z), "+r"(ahead.w));  // before x is looked at
+  }
   return p;
 }
 
@@ -420,8 +433,8 @@ __device__ __forceinline__ Proposal warp_propose(const WalkView& W, const WalkJo
 // Takes the proposal as the walk's next move. Returns false when the walk has
 // ended; `out` is set when the row's open line must be written (RowStage::
 // flush up to row position `pos`).
-template <int APP, int LINE>
-__device__ __forceinline__ bool walk_commit(const WalkJobDev& J, LaneWalk& s, const Proposal& p, int32_t* buf,
+template <int APP, int LINE, bool AHEAD = false>
+__device__ __forceinline__ bool walk_commit(const WalkView& W, const WalkJobDev& J, LaneWalk& s, const Proposal& p, int32_t* buf,
                                             uint32_t& moves, bool& out, uint32_t& pos) {
   const int app = APP >= 0 ? APP : J.app;
   const bool tail = app == APP_PPR && (J.flags & kWalkPprTail);
@@ -441,6 +454,7 @@ __device__ __forceinline__ bool walk_commit(const WalkJobDev& J, LaneWalk& s, co
     s.cur = (uint32_t)p.x;
     ++s.j;
     done = p.stop || (s.j >= L && !tail) || (tail && s.j >= kMaxPprSteps);
+    if (AHEAD && !done) s.R = load_vrec(W, s.cur);
   }
   // A tail walk rewrites its last position until it stops.
   out = done || (at == LINE - 1 && !(tail && pos == L - 1));
