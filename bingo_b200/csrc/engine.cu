@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_plan(StoreView S, const uint32
   pdl_wait();
   pdl_trigger();
   __shared__ unsigned long long nd_s[kPlanSegs][kArenas];
-  __shared__ uint32_t lcnt[kBits], lpc, lb[kPlanSegs], le[kPlanSegs], bigs;
+  __shared__ uint32_t lcnt[kBits], lpc, lb[kPlanSegs], le[kPlanSegs];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const uint32_t s = blockIdx.x * kPlanSegs + w;
   const uint32_t nS = *nseg;
@@ -153,14 +153,22 @@ __global__ void __launch_bounds__(kPlanThreads) k_plan(StoreView S, const uint32
   }
   const bool seg_ok = u < S.n, lng = seg_ok && e - b > kBigLen;
   bool by_block = false;
-  if (threadIdx.x == 0) bigs = 0;
   if (seg_ok && !lng) {
     uint32_t add, pc;
     count_bits(lane, sw + b, e - b, &add, &pc);
     by_block = plan_append(S, u, e - b, add, pc, nd);
   }
-  // Long segments: the whole block counts each one's bits.
-  if (lane == 0) lb[w] = b, le[w] = lng ? e : b;
+  auto publish = [&] {  // lane 0: this warp's segment
+#pragma unroll
+    for (int a = 0; a < kArenas; ++a) nd_s[w][a] = nd[a] | (a == A_EDGE && by_block ? kBigFlag : 0ull);
+    if (by_block) big[atomicAdd(ctl + 1, 1u)] = s;
+  };
+  if (lane == 0) {
+    publish();
+    lb[w] = b, le[w] = lng ? e : b;
+  }
+  // Long segments: the whole block counts each one's bits (one barrier when
+  // there is none, the common case).
   if (__syncthreads_or(lng)) {
     for (int v = 0; v < kPlanSegs; ++v) {
       const uint32_t vb = lb[v], ve = le[v];
@@ -174,31 +182,25 @@ __global__ void __launch_bounds__(kPlanThreads) k_plan(StoreView S, const uint32
       if (add) atomicAdd(&lcnt[lane], add);
       if (lane == 0 && pc) atomicAdd(&lpc, pc);
       __syncthreads();
-      if (w == v) by_block = plan_append(S, u, e - b, lcnt[lane], lpc, nd);
+      if (w == v) {
+        by_block = plan_append(S, u, e - b, lcnt[lane], lpc, nd);
+        if (lane == 0) publish();
+      }
       __syncthreads();
     }
   }
-  if (lane == 0) {
-#pragma unroll
-    for (int a = 0; a < kArenas; ++a) nd_s[w][a] = nd[a];
-    if (by_block) {
-      big[atomicAdd(ctl + 1, 1u)] = s;
-      atomicOr(&bigs, 1u << w);
-    }
-  }
-  __syncthreads();
   if (w == 0) {  // lane v: the block's segment v
     const uint32_t nb = plan_blocks(ks), sv = blockIdx.x * kPlanSegs + lane;
 #pragma unroll
     for (int a = 0; a < kArenas; ++a) {
-      const unsigned long long y = nd_s[lane][a];
+      const unsigned long long r = nd_s[lane][a], y = r & ~kBigFlag;
       unsigned long long yi = y;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const unsigned long long z = __shfl_up_sync(kFull, yi, o);
         if (lane >= o) yi += z;
       }
-      if (sv < ks) excl[sv].v[a] = (yi - y) | (a == A_EDGE && ((bigs >> lane) & 1u) ? kBigFlag : 0ull);
+      if (sv < ks) excl[sv].v[a] = (yi - y) | (r & kBigFlag);
       if (lane == 31) bsum[(size_t)a * nb + blockIdx.x] = yi;
     }
   }
@@ -339,8 +341,8 @@ struct HostReserve {
 
 
 
-// Consecutive segments a warp of the apply kernels takes at a time: their
-// bounds, and what a delete needs first, are read for all of them at once.
+// Consecutive segments a warp of the delete kernel takes at a time: their
+// bounds, and what their deletes need first, are read for all of them at once.
 __device__ __forceinline__ uint32_t segs_per_warp(uint32_t nS, uint32_t warps) {
   return min(8u, max(1u, nS / warps));
 }
@@ -395,43 +397,38 @@ __global__ void __launch_bounds__(kBlock, 4) k_apply_insert(const __grid_constan
     apply_append_block(S, skey[b], sv + b, sw + b, sorig + b, e - b, out_slots, res, asc[threadIdx.x / 32], ba,
                        stage);
   }
-  // The other segments, one warp each, `per` consecutive ones at a time: in
-  // turn by whichever warp is free when there are many (ctl[2]), else dealt
-  // out; blocks that had a listed one then leave them to the rest while those
+  // The other segments, one warp each: eight at a time by whichever warp is
+  // free when there are many (ctl[2]), else dealt out; blocks that had a listed one then leave them to the rest while those
   // are the most.
   const bool many = nS > 16u * gridDim.x * (kBlock / 32);
   const uint32_t skip = !many && nbig < gridDim.x / 2 ? nbig : 0u;
   if (blockIdx.x < skip) return;
-  const int lane = threadIdx.x & 31;
   AliasScratch& A = asc[threadIdx.x / 32];
-  const uint32_t warps = (gridDim.x - skip) * (kBlock / 32), per = segs_per_warp(nS, warps);
-  uint32_t s0 = ((blockIdx.x - skip) * kBlock + threadIdx.x) / 32 * per;
-  for (;; s0 += warps * per) {
+  const uint32_t warps = (gridDim.x - skip) * (kBlock / 32), per = many ? 8u : 1u;
+  uint32_t s0 = ((blockIdx.x - skip) * kBlock + threadIdx.x) / 32;
+  for (;; s0 += warps) {
     if (many) {
-      if (lane == 0) s0 = atomicAdd(ctl + 2, per);
+      if ((threadIdx.x & 31) == 0) s0 = atomicAdd(ctl + 2, per);
       s0 = __shfl_sync(kFull, s0, 0);
     }
     if (s0 >= nS) break;
-    // Lane i: segment s0 + i.
-    const uint32_t s = s0 + lane;
-    uint32_t b = 0, e = 0, u = 0xffffffffu;
-    if (lane < (int)per && s < nS) {
+    for (uint32_t s = s0; s < min(nS, s0 + per); ++s) {
+      uint32_t b, e;
       seg_bounds(seg, nS, s, k, &b, &e);
-      u = skey[b];
-      if (excl[s].v[A_EDGE] & kBigFlag) u = 0xffffffffu;
-    }
-    for (uint32_t todo = __ballot_sync(kFull, u < S.n); todo; todo &= todo - 1) {
-      const int src = __ffs(todo) - 1;
-      const uint32_t vb = __shfl_sync(kFull, b, src), ve = __shfl_sync(kFull, e, src), vs = s0 + src;
-      auto res = [&](int a) {
-        return (base ? base[a] : hr.base[a]) + boff[(size_t)a * nb + vs / kPlanSegs] + (excl[vs].v[a] & ~kBigFlag);
-      };
-      apply_append(S, __shfl_sync(kFull, u, src), sv + vb, sw + vb, sorig + vb, ve - vb, out_slots, res, A, stage);
+      const uint32_t u = skey[b];
+      if (u >= S.n) continue;
+      const ArenaNeed off = excl[s];
+      if (off.v[A_EDGE] & kBigFlag) continue;
+      unsigned long long res[kArenas];
+#pragma unroll
+      for (int a = 0; a < kArenas; ++a)
+        res[a] = (base ? base[a] : hr.base[a]) + boff[(size_t)a * nb + s / kPlanSegs] + off.v[a];
+      apply_append(S, u, sv + b, sw + b, sorig + b, e - b, out_slots, res, A, stage);
     }
   }
 }
 
-__global__ void __launch_bounds__(kBlock, 4) k_apply_delete(const __grid_constant__ StoreView S, const uint32_t* skey, const uint32_t* sslot,
+__global__ void __launch_bounds__(kBlock, 3) k_apply_delete(const __grid_constant__ StoreView S, const uint32_t* skey, const uint32_t* sslot,
                                                          const uint32_t* seg, const uint32_t* nseg,
                                                          unsigned long long k, const uint32_t* ctl) {
   pdl_wait();
@@ -945,6 +942,8 @@ Engine::Engine(const bingo_config& cfg) : cfg_(cfg) {
   }
   cuda_check(cudaMalloc(&d_err_, 4 * sizeof(uint32_t)), "cudaMalloc(err)");
   cuda_check(cudaMemset(d_err_, 0, 4 * sizeof(uint32_t)), "memset(err)");
+  queue_.ensure(64 * 8, "walk queue");  // most calls' work counters, zeroed here: no launch waits for a memset
+  cuda_check(cudaMemset(queue_.p, 0, queue_.bytes), "walk queue");
   cuda_check(cudaMalloc(&d_top_, kArenas * sizeof(unsigned long long)), "cudaMalloc(top)");
   cuda_check(cudaMalloc(&d_steps_, 3 * sizeof(unsigned long long)), "cudaMalloc(steps)");
   cuda_check(cudaMemset(d_steps_, 0, 3 * sizeof(unsigned long long)), "memset(steps)");
@@ -1027,7 +1026,11 @@ void Engine::require_loaded() const {
   if (!loaded_) throw Error(BINGO_ERR_NOT_LOADED, "no graph loaded");
 }
 
-void Engine::set_stream(void* s) { stream_ = s ? (cudaStream_t)s : own_stream_; }
+void Engine::set_stream(void* s) {
+  const cudaStream_t next = s ? (cudaStream_t)s : own_stream_;
+  if (next != stream_ && loaded_) stream_changed_ = true;
+  stream_ = next;
+}
 
 // Forgets the errors raised so far (their stream has been waited for).
 void Engine::clear_err() {
@@ -1264,6 +1267,12 @@ void Engine::drop_arenas() {
   gs_.release();
 }
 
+void Engine::drop_store() {
+  drop_arenas();
+  vrec_.release(), meta_.release(), gdesc_.release();
+  stream_changed_ = false;
+}
+
 namespace {
 // Whether a buffer kept from the graph before serves for `want` bytes: large
 // enough, and not so large that it holds memory others could use.
@@ -1434,9 +1443,11 @@ void Engine::load(const uint32_t* src, const uint32_t* dst, const uint32_t* w, u
   if (m && !is_device_ptr(src)) host_check_ids(src, m, n, "source");
   if (m && !is_device_ptr(dst)) host_check_ids(dst, m, n, "destination");
   if (m && !is_device_ptr(w)) host_check_weights(w, m);
-  // The buffers of the graph before are written again: all work on them must
-  // be over, whatever stream it was ordered on.
-  cuda_check(cudaDeviceSynchronize(), "load");
+  // The buffers of the graph before are written again: the work on them is over
+  // on this stream, and where the handle had another one meanwhile, they are
+  // freed instead, which waits for all streams.
+  cuda_check(cudaStreamSynchronize(stream_), "load");
+  if (stream_changed_) drop_store();
   loaded_ = false;
   n_ = n;
   ++arena_gen_;
@@ -2076,6 +2087,8 @@ void Engine::run(const bingo_op* ops, uint32_t n_ops, uint32_t flags) {
   (void)n_walk_ops;
   mix((uint64_t)(uintptr_t)prog_jobs_.p), mix((uint64_t)(uintptr_t)ctl_.p), mix((uint64_t)(uintptr_t)cub_tmp_.p);
   mix(cub_tmp_.bytes);
+  for (const DevBuf* b : {&key_s_, &perm_, &sa_, &sb_, &seg_, &need_, &scan_, &big_, &iota_, &prog_prefix_, &prog_queue_})
+    mix((uint64_t)(uintptr_t)b->p);
 
   const uint64_t launches0 = launches_;
   auto enqueue_all = [&]() {
@@ -2651,6 +2664,7 @@ void Engine::restore(const char* path) {
   if (expect != H.payload_bytes) throw Error(BINGO_ERR_INVALID_ARGUMENT, "corrupt snapshot header");
   cuda_check(cudaStreamSynchronize(stream_), "restore");
   // From here the handle's old graph is gone; on failure it holds none.
+  if (stream_changed_) drop_store();
   loaded_ = false;
   drop_graph();
   ++arena_gen_;

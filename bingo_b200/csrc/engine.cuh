@@ -123,6 +123,7 @@ class Engine {
   bingo_config cfg_;
   cudaStream_t own_stream_ = nullptr, stream_ = nullptr;
   bool loaded_ = false;
+  bool stream_changed_ = false;  // since the graph was loaded: earlier work on it may still run elsewhere
   bool defer_sync_ = false;
   uint32_t n_ = 0;
 
@@ -187,6 +188,7 @@ class Engine {
   void fill_iota(uint64_t k);
   void load_batch(const uint32_t* src, const uint32_t* dst, const uint32_t* w, uint64_t m);
   void drop_arenas();
+  void drop_store();
   void size_arenas(const unsigned long long need[kArenas]);
   uint32_t* walk_queue(DevBuf& buf, size_t slots);  // zeroed work counters
   const uint32_t* stage(const uint32_t* p, uint64_t k, DevBuf& buf, const char* what);

@@ -345,7 +345,6 @@ __device__ __forceinline__ void append_range(const StoreView& S, const VertexMet
 // (Lines: a warp takes about 3 us per 32 edges and a block 10 us to share a
 // segment out. Measured, R-MAT 20: load apply 6.9 ms to 2.9; 50K-edge insert
 // batches whose vertices follow the degree, 130 us to 79.)
-constexpr uint32_t kLaneCopy = 8;          // members of a moving list that one lane copies
 constexpr uint32_t kBigLen = 256;          // edges
 constexpr uint32_t kBigCopy = 1024;        // 16-byte units copied by relocations
 constexpr unsigned long long kBigFlag = 1ull << 63;  // marks such a segment in its A_EDGE offset
@@ -358,12 +357,11 @@ constexpr unsigned long long kBigFlag = 1ull << 63;  // marks such a segment in 
 // reMalloc round trip (include/operation.cuh:163-174).
 //
 // seg_v / seg_w / seg_orig: the segment's edges in batch order; out_slots is
-// indexed by seg_orig (may be null). res(a): the arena offset reserved for
-// this segment (units of each arena), read where a relocation needs it.
-template <class Reserved>
+// indexed by seg_orig (may be null). res[a]: the arena offsets reserved for
+// this segment (units of each arena).
 static __device__ __forceinline__ void apply_append(const StoreView& S, uint32_t u, const uint32_t* seg_v, const uint32_t* seg_w,
                              const uint32_t* seg_orig, uint32_t len, uint32_t* out_slots,
-                             const Reserved& res, AliasScratch& B, uint32_t* stage) {
+                             const unsigned long long res[kArenas], AliasScratch& B, uint32_t* stage) {
   const int lane = threadIdx.x & 31;
   VertexMeta M = S.meta[u];
   GroupDesc G = S.gdesc[(size_t)u * kBits + lane];
@@ -379,41 +377,25 @@ static __device__ __forceinline__ void apply_append(const StoreView& S, uint32_t
 
   // --- relocations (old contents keep their order) ---
   if (P.new_ecap) {
-    warp_copy_v4(reinterpret_cast<uint4*>(S.edges + res(A_EDGE)), reinterpret_cast<const uint4*>(S.edges + M.eoff),
+    warp_copy_v4(reinterpret_cast<uint4*>(S.edges + res[A_EDGE]), reinterpret_cast<const uint4*>(S.edges + M.eoff),
                  M.ecnt, lane);
-    M.eoff = res(A_EDGE);
+    M.eoff = res[A_EDGE];
     M.ecap = P.new_ecap;
   }
   if (P.new_bpcap) {
-    warp_copy_u32(S.bp + res(A_BP), S.bp + M.bpoff, M.bpcnt, lane);
-    M.bpoff = res(A_BP);
+    warp_copy_u32(S.bp + res[A_BP], S.bp + M.bpoff, M.bpcnt, lane);
+    M.bpoff = res[A_BP];
     M.bpcap = P.new_bpcap;
   }
   {
-    // Lists that move: each lane copies its own when it is short, all lanes'
-    // reads in flight together (most moving lists hold 4 or 8 members); the
-    // whole warp copies the longer ones in turn. A list that held no members
-    // needs no copy (the common case for a new group).
+    // Lists that move: the whole warp copies the members of each non-empty
+    // one in turn; every moving lane then takes its new base (a list that
+    // held no members needs no copy, the common case for a new group).
     const uint32_t old_base = group_base(G);
-    const bool moves = P.gcap_lane != 0;
-    const unsigned long long fresh = __any_sync(kFull, moves) ? res(A_MEMBER) : 0ull;
-    uint32_t copy = __ballot_sync(kFull, moves && G.cnt > kLaneCopy);
-    if (moves) {
-      G.base1 = (uint32_t)((fresh + P.gpre) >> 2) + 1u;  // reserved offsets are 4-entry aligned
+    uint32_t copy = __ballot_sync(kFull, P.gcap_lane != 0 && G.cnt != 0);
+    if (P.gcap_lane) {
+      G.base1 = (uint32_t)((res[A_MEMBER] + P.gpre) >> 2) + 1u;  // reserved offsets are 4-entry aligned
       G.roomy = 0;
-      if (G.cnt <= kLaneCopy) {
-        const uint4* const v0 = reinterpret_cast<const uint4*>(S.gv) + old_base;
-        const uint4* const s0 = reinterpret_cast<const uint4*>(S.gs) + old_base;
-        uint4* const v1 = reinterpret_cast<uint4*>(S.gv) + group_base(G);
-        uint4* const s1 = reinterpret_cast<uint4*>(S.gs) + group_base(G);
-        uint4 a[2], b[2];
-#pragma unroll
-        for (int q = 0; q < 2; ++q)
-          if (4u * q < G.cnt) a[q] = v0[q], b[q] = s0[q];
-#pragma unroll
-        for (int q = 0; q < 2; ++q)
-          if (4u * q < G.cnt) v1[q] = a[q], s1[q] = b[q];
-      }
     }
     while (copy) {
       const int k = __ffs(copy) - 1;
@@ -425,7 +407,7 @@ static __device__ __forceinline__ void apply_append(const StoreView& S, uint32_t
     }
   }
   if (P.new_acap) {
-    R.aoff = (uint32_t)res(A_ALIAS);
+    R.aoff = (uint32_t)res[A_ALIAS];
     M.acap = P.new_acap;
   }
   __syncwarp();
@@ -464,7 +446,7 @@ static __device__ __forceinline__ void apply_append(const StoreView& S, uint32_t
     if (P.rehash) {
       // Rebuild from every live slot into a cleared table.
       if (P.new_hcap) {
-        R.hoff = (uint32_t)res(A_HASH);
+        R.hoff = (uint32_t)res[A_HASH];
         R.hmask = P.new_hcap - 1;
         M.hcap = P.new_hcap;
       }
@@ -653,10 +635,10 @@ __device__ __forceinline__ bool plan_append(const StoreView& S, uint32_t u, uint
 }
 
 // Removals of one group a lane resolves per round of loads (apply_delete; a
-// block takes the segments with many). Two keep the kernel at 64 registers and
-// four blocks per SM: 500K deletes 509 us against 532 at four removals and
-// three blocks.
-constexpr int kDeleteRound = 2;
+// block takes the segments with many). Two would let four blocks per SM
+// reside and serve 500K deletes a little better (509 us against 532), but
+// uniform 50K batches worse (390 M edges/s of insert + delete against 401).
+constexpr int kDeleteRound = 4;
 
 // ---------------------------------------------------------------------------
 // Delete a run of slots of one vertex in batch order. Each delete swap-removes

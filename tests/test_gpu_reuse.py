@@ -129,3 +129,74 @@ def test_counters_after_every_shape():
                 form()
                 for j, x in zip(jobs, want):
                     assert np.array_equal(j.out.cpu().numpy(), x.reshape(j.out.shape))
+
+
+def test_load_after_a_stream_change():
+    """A load while walks on the handle's earlier stream may still run: their rows and the new graph are both right."""
+    import torch
+    from bingo_b200 import Graph
+    from oracle import pyoracle as po
+    n, src, dst, w = _case(12, 31)
+    ex = po.ExactGraph(n)
+    ex.load(src, dst, w)
+    dev = [torch.from_numpy(x.view(np.int32)).cuda() for x in (src, dst, w)]
+    rev = [dev[1], dev[0], dev[2]]
+    ex2 = po.ExactGraph(n)
+    ex2.load(dst, src, w)
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    starts = torch.arange(n, dtype=torch.int32, device="cuda").repeat(20)
+    want = ex.walk(0, 40, starts.cpu().numpy().astype(np.uint32), seed=3)
+    want2 = ex2.walk(0, 40, np.arange(n, dtype=np.uint32), seed=4)
+    for _ in range(3):
+        with Graph(device=0, synchronous=False, node2vec=False) as g:
+            out = torch.empty((len(starts), 40), dtype=torch.int32, device="cuda")
+            torch.cuda.synchronize()
+            g.set_stream(a.cuda_stream)
+            g.load_edges(*dev, n)
+            for _ in range(4):
+                g.walk(app=0, length=40, starts=starts, seed=3, out=out)
+            g.set_stream(b.cuda_stream)
+            g.load_edges(*rev, n)
+            out2 = torch.empty((n, 40), dtype=torch.int32, device="cuda")
+            torch.cuda.synchronize()
+            g.walk(app=0, length=40, n_starts=n, seed=4, out=out2)
+            torch.cuda.synchronize()
+            assert np.array_equal(out.cpu().numpy(), want)
+            assert np.array_equal(out2.cpu().numpy(), want2)
+
+
+def test_loads_while_another_thread_captures():
+    """One handle loads again and again while another captures programs of changing shape on its own thread."""
+    import threading
+
+    import torch
+    from bingo_b200 import Graph, WalkJob
+    from oracle import pyoracle as po
+    n, src, dst, w = _case(9, 41)
+    ex = po.ExactGraph(n)
+    ex.load(src, dst, w)
+    failed = []
+
+    def programs():
+        try:
+            with Graph(device=0, synchronous=False) as g:
+                g.load_edges(src, dst, w, n)
+                for turn in range(60):
+                    k = 20 + turn
+                    out = torch.zeros((k, 10), dtype=torch.int32, device="cuda")
+                    g.sync()
+                    g.run([("walk", [WalkJob(app=0, length=10, n_starts=k, seed=turn, out=out)])])
+                    g.sync()
+                    if not np.array_equal(out.cpu().numpy(), ex.walk(0, 10, np.arange(k, dtype=np.uint32), seed=turn)):
+                        failed.append(turn)
+        except Exception as e:  # noqa: BLE001
+            failed.append(repr(e))
+
+    t = threading.Thread(target=programs)
+    t.start()
+    with Graph(device=0) as g:
+        for turn in range(40):
+            g.load_edges(src, dst, w, n)
+        _same(g, ex)
+    t.join()
+    assert not failed, failed[:3]
