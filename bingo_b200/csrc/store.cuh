@@ -807,7 +807,7 @@ static __device__ void apply_delete(const StoreView& S, uint32_t u, const uint32
 // the removals of its group a few per round trip, so a hub's deletes were a
 // chain that set the kernel's time (50K deletes on R-MAT 20: 116 of vertex 0,
 // 55 of them in one group; 500K: over a thousand). 500K deletes with the
-// grouping: 632 us, 509 with this and the reads below brought near.
+// grouping: 632 us, 532 with this and the reads of k_apply_delete brought near.
 constexpr uint32_t kBigDelete = 24;
 
 constexpr int kDeleteWarps = 8;  // warps of a block that deletes one segment
