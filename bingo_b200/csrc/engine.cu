@@ -562,8 +562,9 @@ __global__ void __launch_bounds__(kBlock) k_pair_slots(StoreView S, const unsign
 
 // Persistent walk kernel with per-lane refill. Each warp owns a range of
 // walk items and hands them to idle lanes; when the range runs out it pulls
-// the next `chunk` items from one device counter (queue[0], zero at launch
-// and zeroed again by the last warp to finish, which queue[1] counts). MULTI = false: every item is a walk of the single job J0.
+// the next `chunk` items from one device counter (WalkQueue, zero at launch
+// and zeroed again by the last warp to finish). MULTI = false: every item is
+// a walk of the single job J0.
 // MULTI = true: items index the concatenated jobs of a device job table
 // (prefix = running walk counts) and each lane follows its own job; APP >= 0
 // when every job of the table has that app, APP < 0 for a mixed table.
@@ -598,7 +599,7 @@ __device__ __forceinline__ uint32_t job_of_item(const uint32_t* __restrict__ pre
 template <int APP, bool MULTI>
 __global__ void __launch_bounds__(kBlock, walk_min_blocks(APP))
     k_walk(WalkView W, WalkJobDev J0, const WalkJobDev* __restrict__ jobs, const uint32_t* __restrict__ prefix,
-           uint32_t n_jobs, uint32_t total, uint32_t* queue, uint32_t chunk) {
+           uint32_t n_jobs, uint32_t total, WalkQueue* queue, uint32_t chunk) {
   constexpr int kLine = walk_line(APP);
   using Stage = RowStage<kLine>;
   constexpr bool kRows = APP != APP_SAMPLING;                   // sampling jobs write no rows
@@ -624,22 +625,20 @@ __global__ void __launch_bounds__(kBlock, walk_min_blocks(APP))
   const uint32_t warps = gridDim.x * (kBlock / 32);
   // A small launch's walks spread over all its warps (walks that take trials
   // spread inside theirs).
-  const uint32_t lanes = kTrials ? 32u : min(32u, (total + warps - 1) / warps);
+  const uint32_t lanes = kTrials ? 32u : min(32u, walk_share(total, warps));
   for (;;) {
     uint32_t idle = drained ? 0u : __ballot_sync(kFull, !active);
     uint32_t room = 0;
     if (idle) room = lanes - min(lanes, 32u - __popc(idle));
     while (idle && room && !drained) {
       if (wb >= we) {
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(queue, chunk);
-        base = __shfl_sync(kFull, base, 0);
-        if (base >= total) {
+        unsigned long long base = 0;
+        if (lane == 0) base = min(atomicAdd(&queue->next, (unsigned long long)chunk), (unsigned long long)total);
+        base = __shfl_sync(kFull, (uint32_t)base, 0);
+        if (!claim_range(base, total, chunk, &wb, &we)) {
           drained = true;
           break;
         }
-        wb = base;
-        we = base + min(chunk, total - base);
       }
       const uint32_t take = min(min((uint32_t)__popc(idle), room), we - wb);
       room -= take;
@@ -682,7 +681,7 @@ __global__ void __launch_bounds__(kBlock, walk_min_blocks(APP))
   add_steps(W, moves);
   add_n2v(W, s);
   // The last warp leaves the work counter zeroed for the next launch.
-  if (lane == 0 && atomicAdd(queue + 1, 1u) + 1 == warps) queue[0] = queue[1] = 0;
+  if (lane == 0 && atomicAdd(&queue->done, 1u) + 1 == warps) queue->next = 0, queue->done = 0;
 }
 
 __global__ void k_philox(const uint32_t* ctr, unsigned long long count, uint32_t k0, uint32_t k1, uint32_t* out) {
@@ -733,7 +732,7 @@ uint32_t walk_chunk_of(const Tuning& t, int app, uint32_t total, unsigned grid) 
   if (t.walk_chunk) return t.walk_chunk;
   const uint32_t warps = grid * (kBlock / 32);
   const bool one_fill = app != APP_NODE2VEC && app >= 0 && total <= 32ull * warps;  // every warp claims its share at once
-  return one_fill ? (total + warps - 1) / warps : walk_default_chunk(app);
+  return one_fill ? walk_share(total, warps) : walk_default_chunk(app);
 }
 
 // Blocks of a walk launch: one resident wave at most, and at least
@@ -748,7 +747,7 @@ unsigned walk_grid(unsigned long long total, const Tuning& t) {
 
 template <int APP, bool MULTI>
 void launch_walk(cudaStream_t st, const WalkView& W, const WalkJobDev& J0, const WalkJobDev* jobs,
-                 const uint32_t* prefix, uint32_t n_jobs, uint32_t total, uint32_t* queue, const Tuning& t) {
+                 const uint32_t* prefix, uint32_t n_jobs, uint32_t total, WalkQueue* queue, const Tuning& t) {
   const unsigned grid = walk_grid<APP, MULTI>(total, t);
   k_walk<APP, MULTI><<<grid, kBlock, 0, st>>>(W, J0, jobs, prefix, n_jobs, total, queue,
                                               walk_chunk_of(t, APP, total, grid));
@@ -757,7 +756,7 @@ void launch_walk(cudaStream_t st, const WalkView& W, const WalkJobDev& J0, const
 // Launches the persistent walk kernel for a device job table whose jobs all
 // have app `app` (or any app when app < 0).
 void launch_walk_table(cudaStream_t st, int app, const WalkView& W, const WalkJobDev& J0, const WalkJobDev* jobs,
-                       const uint32_t* prefix, uint32_t n_jobs, uint32_t total, uint32_t* queue, const Tuning& t) {
+                       const uint32_t* prefix, uint32_t n_jobs, uint32_t total, WalkQueue* queue, const Tuning& t) {
   auto* go = app == APP_DEEPWALK   ? launch_walk<APP_DEEPWALK, true>
              : app == APP_NODE2VEC ? launch_walk<APP_NODE2VEC, true>
              : app == APP_PPR      ? launch_walk<APP_PPR, true>
@@ -768,7 +767,7 @@ void launch_walk_table(cudaStream_t st, int app, const WalkView& W, const WalkJo
 }
 
 // One job's walks (the plain form).
-void launch_walk_job(cudaStream_t st, const WalkView& W, const WalkJobDev& J, uint32_t* queue, const Tuning& t) {
+void launch_walk_job(cudaStream_t st, const WalkView& W, const WalkJobDev& J, WalkQueue* queue, const Tuning& t) {
   auto* go = J.app == APP_DEEPWALK   ? launch_walk<APP_DEEPWALK, false>
              : J.app == APP_NODE2VEC ? launch_walk<APP_NODE2VEC, false>
              : J.app == APP_PPR      ? launch_walk<APP_PPR, false>
@@ -942,7 +941,7 @@ Engine::Engine(const bingo_config& cfg) : cfg_(cfg) {
   }
   cuda_check(cudaMalloc(&d_err_, 4 * sizeof(uint32_t)), "cudaMalloc(err)");
   cuda_check(cudaMemset(d_err_, 0, 4 * sizeof(uint32_t)), "memset(err)");
-  queue_.ensure(64 * 8, "walk queue");  // most calls' work counters, zeroed here: no launch waits for a memset
+  queue_.ensure(64 * sizeof(WalkQueue), "walk queue");  // most calls' work counters, zeroed here: no launch waits for a memset
   cuda_check(cudaMemset(queue_.p, 0, queue_.bytes), "walk queue");
   cuda_check(cudaMalloc(&d_top_, kArenas * sizeof(unsigned long long)), "cudaMalloc(top)");
   cuda_check(cudaMalloc(&d_steps_, 3 * sizeof(unsigned long long)), "cudaMalloc(steps)");
@@ -1109,15 +1108,15 @@ void Engine::ensure_batch_scratch(uint64_t k) {
   group_cluster_ok();  // probed here, outside any stream capture
 }
 
-// `slots` work counters of walk launches, two words each (next item, warps
-// done). Zeroed when allocated; every launch leaves its own zeroed.
-uint32_t* Engine::walk_queue(DevBuf& buf, size_t slots) {
-  const size_t want = slots * 8;
+// `slots` work counters of walk launches. Zeroed when allocated; every launch
+// leaves its own zeroed.
+WalkQueue* Engine::walk_queue(DevBuf& buf, size_t slots) {
+  const size_t want = slots * sizeof(WalkQueue);
   if (!buf.p || buf.bytes < want) {
     buf.ensure(want, "walk queue");
     cuda_check(cudaMemsetAsync(buf.p, 0, buf.bytes, stream_), "walk queue");
   }
-  return buf.as<uint32_t>();
+  return buf.as<WalkQueue>();
 }
 
 const uint32_t* Engine::stage(const uint32_t* p, uint64_t k, DevBuf& buf, const char* what) {
@@ -1836,12 +1835,12 @@ void Engine::walk(const bingo_walk_job* jobs, uint32_t n_jobs, uint32_t mode) {
       throw Error(BINGO_ERR_INVALID_ARGUMENT, "device output must be 32-byte aligned");
   }
   const WalkView W = wview();
-  uint32_t* q = walk_queue(queue_, std::max<uint32_t>(n_jobs, 4));
+  WalkQueue* q = walk_queue(queue_, std::max<uint32_t>(n_jobs, 4));
   if (mode == BINGO_WALK_PLAIN) {
     // One launch per job, each with its own work counter.
     for (uint32_t j = 0; j < n_jobs; ++j) {
       if (!dj[j].n) continue;
-      launch_walk_job(stream_, W, dj[j], q + 2 * j, tuning_);
+      launch_walk_job(stream_, W, dj[j], q + j, tuning_);
       ++launches_;
     }
   } else if (prefix[n_jobs]) {
@@ -1859,7 +1858,7 @@ void Engine::walk(const bingo_walk_job* jobs, uint32_t n_jobs, uint32_t mode) {
     for (size_t gi = 0; gi < groups.size(); ++gi) {
       const WalkGroup& G = groups[gi];
       launch_walk_table(stream_, G.app, W, table[G.job_off], jobs_.as<WalkJobDev>() + G.job_off,
-                        prefix_.as<uint32_t>() + G.pf_off, G.n_jobs, G.total, q + 2 * gi, tuning_);
+                        prefix_.as<uint32_t>() + G.pf_off, G.n_jobs, G.total, q + gi, tuning_);
       ++launches_;
     }
   }
@@ -2076,7 +2075,7 @@ void Engine::run(const bingo_op* ops, uint32_t n_ops, uint32_t flags) {
   // Job tables are read by the walk kernels from device memory, so their
   // contents may change between replays of a captured program.
   if (!table.empty()) {
-    const size_t jb = table.size() * sizeof(WalkJobDev), pb = pf.size() * 4, qb = groups.size() * 8;
+    const size_t jb = table.size() * sizeof(WalkJobDev), pb = pf.size() * 4, qb = groups.size() * sizeof(WalkQueue);
     if (jb > prog_jobs_.bytes || pb > prog_prefix_.bytes || qb > prog_queue_.bytes) drop_graph();
     prog_jobs_.ensure(jb, "program jobs");
     prog_prefix_.ensure(pb, "program jobs");
@@ -2107,7 +2106,7 @@ void Engine::run(const bingo_op* ops, uint32_t n_ops, uint32_t flags) {
           const WalkGroup& G = groups[gi];
           launch_walk_table(stream_, G.app, W, table[G.job_off], prog_jobs_.as<WalkJobDev>() + G.job_off,
                             prog_prefix_.as<uint32_t>() + G.pf_off, G.n_jobs, G.total,
-                            prog_queue_.as<uint32_t>() + 2 * gi, tuning_);
+                            prog_queue_.as<WalkQueue>() + gi, tuning_);
           ++launches_;
         }
       }
@@ -2153,7 +2152,7 @@ constexpr uint32_t kNoAllocMaxJobs = 64;
 struct NoAllocScratch {
   WalkJobDev jobs[kNoAllocMaxJobs];
   uint32_t prefix[kNoAllocMaxJobs + 1];
-  uint32_t queue[2];
+  WalkQueue queue;
 };
 static __device__ __align__(256) unsigned char g_noalloc_scratch[sizeof(NoAllocScratch)];
 
@@ -2174,7 +2173,7 @@ __global__ void k_noalloc_stage(const __grid_constant__ NoAllocJobs in, NoAllocS
   uint32_t* out = reinterpret_cast<uint32_t*>(dst->jobs);
   for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) out[i] = src[i];
   for (uint32_t i = threadIdx.x; i <= in.n_jobs; i += blockDim.x) dst->prefix[i] = in.prefix[i];
-  if (threadIdx.x == 0) dst->queue[0] = dst->queue[1] = 0;
+  if (threadIdx.x == 0) dst->queue = WalkQueue{0, 0, 0};
 }
 static_assert(sizeof(WalkJobDev) % 4 == 0, "word copy");
 
@@ -2257,7 +2256,7 @@ void Engine::walk_noalloc(const bingo_walk_job* jobs, uint32_t n_jobs) {
   cuda_check(cudaGetLastError(), "no-alloc job staging");
   ++launches_;
   const WalkView W = wview();
-  launch_walk_table(stream_, -1, W, dj[0], scratch->jobs, scratch->prefix, n_jobs, (uint32_t)total, scratch->queue,
+  launch_walk_table(stream_, -1, W, dj[0], scratch->jobs, scratch->prefix, n_jobs, (uint32_t)total, &scratch->queue,
                     tuning_);
   ++launches_;
   finish_call();

@@ -11,6 +11,7 @@
 #include <nvtx3/nvToolsExt.h>
 
 #include "../../include/bingo.h"
+#include "claim.h"
 #include "common.cuh"
 #include "walk.cuh"
 
@@ -190,7 +191,7 @@ class Engine {
   void drop_arenas();
   void drop_store();
   void size_arenas(const unsigned long long need[kArenas]);
-  uint32_t* walk_queue(DevBuf& buf, size_t slots);  // zeroed work counters
+  WalkQueue* walk_queue(DevBuf& buf, size_t slots);  // zeroed work counters
   const uint32_t* stage(const uint32_t* p, uint64_t k, DevBuf& buf, const char* what);
   // Stable grouping of a batch by `key` into key_s_/perm_/sa_/sb_/seg_/nseg_,
   // with the batch status word zeroed and the batch validated (`insert`: the
