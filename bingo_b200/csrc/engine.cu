@@ -1028,6 +1028,7 @@ void Engine::require_loaded() const {
 void Engine::set_stream(void* s) {
   const cudaStream_t next = s ? (cudaStream_t)s : own_stream_;
   if (next != stream_ && loaded_) stream_changed_ = true;
+  if (next != stream_ && walks_pending_) counters_shared_ = true;
   stream_ = next;
 }
 
@@ -1039,6 +1040,7 @@ void Engine::clear_err() {
 
 int Engine::sync() {
   cuda_check(cudaStreamSynchronize(stream_), "stream synchronize");
+  walks_pending_ = false;
   cuda_check(cudaStreamSynchronize(xstream_), "result copies");
   // The copy of the error words costs about 8 us, more than a small call's
   // kernels: it is made only when the device raised the flag.
@@ -1109,7 +1111,7 @@ void Engine::ensure_batch_scratch(uint64_t k) {
 }
 
 // `slots` work counters of walk launches. Zeroed when allocated; every launch
-// leaves its own zeroed.
+// leaves its own zeroed (zero_counters).
 WalkQueue* Engine::walk_queue(DevBuf& buf, size_t slots) {
   const size_t want = slots * sizeof(WalkQueue);
   if (!buf.p || buf.bytes < want) {
@@ -1117,6 +1119,18 @@ WalkQueue* Engine::walk_queue(DevBuf& buf, size_t slots) {
     cuda_check(cudaMemsetAsync(buf.p, 0, buf.bytes, stream_), "walk queue");
   }
   return buf.as<WalkQueue>();
+}
+
+// Before launches that use the first `slots` counters of buf. A launch that
+// ran alone has left its counter zeroed, and a memset would cost a small call
+// 2 us; but where launches of this handle may overlap (the stream was changed
+// with walks in flight, or the caller captures this launch and replays it
+// beside others), one can leave a count behind that every later launch would
+// start from, so each then starts from zero as if it were the first.
+void Engine::zero_counters(DevBuf& buf, size_t slots) {
+  walks_pending_ = true;
+  if (counters_shared_)
+    cuda_check(cudaMemsetAsync(buf.p, 0, slots * sizeof(WalkQueue), stream_), "walk queue reset");
 }
 
 const uint32_t* Engine::stage(const uint32_t* p, uint64_t k, DevBuf& buf, const char* what) {
@@ -1836,6 +1850,12 @@ void Engine::walk(const bingo_walk_job* jobs, uint32_t n_jobs, uint32_t mode) {
   }
   const WalkView W = wview();
   WalkQueue* q = walk_queue(queue_, std::max<uint32_t>(n_jobs, 4));
+  if (!cfg_.synchronous && !counters_shared_) {  // (a synchronous call cannot be captured)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    cuda_check(cudaStreamIsCapturing(stream_, &cap), "capture status");
+    counters_shared_ = cap != cudaStreamCaptureStatusNone;
+  }
+  zero_counters(queue_, n_jobs);
   if (mode == BINGO_WALK_PLAIN) {
     // One launch per job, each with its own work counter.
     for (uint32_t j = 0; j < n_jobs; ++j) {
@@ -2026,7 +2046,7 @@ void Engine::run(const bingo_op* ops, uint32_t n_ops, uint32_t flags) {
   std::vector<size_t> grp_begin(n_ops, 0), grp_end(n_ops, 0);
   const bool split = tuning_.walk_split != 0;
   mix(tuning_.walk_chunk), mix(tuning_.walk_blocks_per_sm), mix(tuning_.walk_split), mix(tuning_.walk_order);
-  mix(tuning_.apply_blocks_per_sm);
+  mix(tuning_.apply_blocks_per_sm), mix(counters_shared_);
   dj.reserve(n_jobs_total);
   for (uint32_t i = 0; i < n_ops; ++i) {
     const bingo_op& o = ops[i];
@@ -2091,6 +2111,7 @@ void Engine::run(const bingo_op* ops, uint32_t n_ops, uint32_t flags) {
 
   const uint64_t launches0 = launches_;
   auto enqueue_all = [&]() {
+    if (!groups.empty()) zero_counters(prog_queue_, groups.size());
     const WalkView W = wview();
     for (uint32_t i = 0; i < n_ops; ++i) {
       const bingo_op& o = ops[i];
@@ -2132,6 +2153,7 @@ void Engine::run(const bingo_op* ops, uint32_t n_ops, uint32_t flags) {
       launches_ = launches0;
     }
     cuda_check(cudaGraphLaunch(graph_exec_, stream_), "graph launch");
+    if (!groups.empty()) walks_pending_ = true;
     launches_ += graph_launches_;
   } else {
     enqueue_all();

@@ -125,6 +125,8 @@ class Engine {
   cudaStream_t own_stream_ = nullptr, stream_ = nullptr;
   bool loaded_ = false;
   bool stream_changed_ = false;  // since the graph was loaded: earlier work on it may still run elsewhere
+  bool walks_pending_ = false;    // walk launches since the stream was last waited for
+  bool counters_shared_ = false;  // work counters may be used by overlapping launches (zero_counters)
   bool defer_sync_ = false;
   uint32_t n_ = 0;
 
@@ -192,6 +194,7 @@ class Engine {
   void drop_store();
   void size_arenas(const unsigned long long need[kArenas]);
   WalkQueue* walk_queue(DevBuf& buf, size_t slots);  // zeroed work counters
+  void zero_counters(DevBuf& buf, size_t slots);
   const uint32_t* stage(const uint32_t* p, uint64_t k, DevBuf& buf, const char* what);
   // Stable grouping of a batch by `key` into key_s_/perm_/sa_/sb_/seg_/nseg_,
   // with the batch status word zeroed and the batch validated (`insert`: the

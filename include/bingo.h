@@ -415,7 +415,9 @@ int bingo_serve_stop(bingo_handle* h);
 int bingo_sync(bingo_handle* h);
 
 /* The CUDA stream calls are ordered on (cudaStream_t as void*); NULL restores
- * the handle's own stream. */
+ * the handle's own stream. All calls of a handle share its scratch: where an
+ * asynchronous handle still has work on the stream before, the caller orders
+ * that work before the calls that follow (an event, or a wait). */
 int bingo_set_stream(bingo_handle* h, void* stream);
 
 int bingo_get_stats(bingo_handle* h, bingo_stats* out);
