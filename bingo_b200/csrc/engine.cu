@@ -103,14 +103,19 @@ __global__ void k_validate(const uint32_t* a, const uint32_t* b, const uint32_t*
 }
 
 // Sorted order -> payload columns in sorted order + segment heads.
+// `over` > 0: the positions of segments longer than that are listed in
+// big[0..ctl[1]), in no particular order.
 __global__ void k_gather(const uint32_t* key, const uint32_t* perm, const uint32_t* a, const uint32_t* b,
-                         uint32_t* sa, uint32_t* sb, uint8_t* head, unsigned long long k) {
+                         uint32_t* sa, uint32_t* sb, uint8_t* head, unsigned long long k, uint32_t over,
+                         uint32_t* big, uint32_t* ctl) {
   for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < k;
        i += (unsigned long long)gridDim.x * blockDim.x) {
     const uint32_t p = perm[i];
     sa[i] = a[p];
     if (b) sb[i] = b[p];
-    head[i] = (i == 0 || key[i] != key[i - 1]) ? 1 : 0;
+    const bool h = i == 0 || key[i] != key[i - 1];
+    head[i] = h;
+    if (h && over && i + over < k && key[i + over] == key[i]) big[atomicAdd(ctl + 1, 1u)] = (uint32_t)i;
   }
 }
 
@@ -430,35 +435,30 @@ __global__ void __launch_bounds__(kBlock, 4) k_apply_insert(const __grid_constan
 
 __global__ void __launch_bounds__(kBlock, 3) k_apply_delete(const __grid_constant__ StoreView S, const uint32_t* skey, const uint32_t* sslot,
                                                          const uint32_t* seg, const uint32_t* nseg,
-                                                         unsigned long long k, const uint32_t* ctl) {
+                                                         unsigned long long k, const uint32_t* ctl,
+                                                         const uint32_t* big) {
   pdl_wait();
   pdl_trigger();
   static_assert(kBlock / 32 == kDeleteWarps, "a block deletes a long segment");
   __shared__ AliasScratch asc[kBlock / 32];
   __shared__ uint32_t stage[kBlock / 32][64];
   __shared__ BlockDelete bd;
-  __shared__ uint32_t llist[kBlock], nlong;
   if (*ctl) return;
-  const uint32_t nS = *nseg;
-  // Long segments, a block each: every block looks through its share (spread,
-  // since the hubs of a skewed graph are neighbours).
-  for (uint32_t t0 = 0; t0 < nS; t0 += gridDim.x * kBlock) {
-    if (threadIdx.x == 0) nlong = 0;
-    __syncthreads();
-    const uint32_t s = t0 + blockIdx.x + gridDim.x * threadIdx.x;
-    uint32_t b, e;
-    if (s < nS) {
-      seg_bounds(seg, nS, s, k, &b, &e);
-      if (e - b > kBigDelete && skey[b] < S.n) llist[atomicAdd(&nlong, 1u)] = s;
-    }
-    __syncthreads();
-    for (uint32_t q = 0; q < nlong; ++q) {
-      seg_bounds(seg, nS, llist[q], k, &b, &e);
-      apply_delete_block(S, skey[b], sslot + b, e - b, asc[threadIdx.x / 32], bd);
-    }
-    __syncthreads();
+  const uint32_t nS = *nseg, nlong = ctl[1];
+  // Long segments, a block each, from the list that the grouping made of their
+  // positions (k_gather, k_group_small). Every block looking through the
+  // segments for them instead cost a uniform batch of 50K 10 us of 249.
+  for (uint32_t q = blockIdx.x; q < nlong; q += gridDim.x) {
+    const uint32_t b = big[q], u = skey[b];
+    uint32_t len = 0, n;
+    do {
+      const unsigned long long p = (unsigned long long)b + len + threadIdx.x;
+      n = __syncthreads_count(p < k && skey[p] == u);
+      len += n;
+    } while (n == kBlock);
+    if (u < S.n) apply_delete_block(S, u, sslot + b, len, asc[threadIdx.x / 32], bd);
   }
-  // The others, as in k_apply_insert.
+  // The others, one warp each, up to eight consecutive ones at a time.
   const int lane = threadIdx.x & 31;
   AliasScratch& A = asc[threadIdx.x / 32];
   const uint32_t warps = gridDim.x * (kBlock / 32), per = segs_per_warp(nS, warps);
@@ -1179,13 +1179,14 @@ bool group_kernel_ready() {
 template <int CTAS, int IPT>
 cudaError_t launch_group(cudaStream_t s, const uint32_t* key, const uint32_t* a, const uint32_t* b, uint32_t k,
                          uint32_t n, int end_bit, bool insert, uint32_t* key_s, uint32_t* perm, uint32_t* sa,
-                         uint32_t* sb, uint32_t* seg, uint32_t* nseg, uint32_t* ctl, uint32_t* err) {
+                         uint32_t* sb, uint32_t* seg, uint32_t* nseg, uint32_t* ctl, uint32_t* err, uint32_t over,
+                         uint32_t* big) {
   const uint32_t ipt = group_ipt(k, CTAS);
   cudaLaunchConfig_t lc;
   cudaLaunchAttribute at[2];
   group_launch_config(lc, at, CTAS, ipt, s);
   return cudaLaunchKernelEx(&lc, k_group_small<CTAS, IPT>, key, a, b, k, n, end_bit, ipt, insert ? 1 : 0, key_s,
-                            perm, sa, sb, seg, nseg, ctl, err);
+                            perm, sa, sb, seg, nseg, ctl, err, over, big);
 }
 }  // namespace
 
@@ -1202,13 +1203,14 @@ int Engine::group_cluster_ok() {
 void Engine::group_by_vertex(const uint32_t* key, const uint32_t* a, const uint32_t* b, uint64_t k, bool insert) {
   int end_bit = 1;
   while (end_bit < 32 && (1ull << end_bit) < n_) ++end_bit;
+  const uint32_t over = insert ? 0 : kBigDelete;  // deletes: list the segments longer than this (inserts: k_plan does)
   const int gc = k >= 1 && k <= kGroupMax ? group_cluster_ok() : 0;
   const bool small = (gc & 1) && (k <= kGroupSmallMax || (!(gc & 2) && k <= 8ull * kGroupThreads * kGroupIptSmall));
   if (small || (gc & 2)) {
     auto* launch = small ? launch_group<8, kGroupIptSmall> : launch_group<16, kGroupIptLarge>;
     cuda_check(launch(stream_, key, a, b, (uint32_t)k, n_, end_bit, insert, key_s_.as<uint32_t>(),
                       perm_.as<uint32_t>(), sa_.as<uint32_t>(), sb_.as<uint32_t>(), seg_.as<uint32_t>(),
-                      nseg_.as<uint32_t>(), ctl_.as<uint32_t>(), d_err_),
+                      nseg_.as<uint32_t>(), ctl_.as<uint32_t>(), d_err_, over, big_.as<uint32_t>()),
                "group batch");
     ++launches_;
     return;
@@ -1224,7 +1226,8 @@ void Engine::group_by_vertex(const uint32_t* key, const uint32_t* a, const uint3
              "radix sort");
   k_gather<<<grid_for(k, kBlock, 16), kBlock, 0, stream_>>>(key_s_.as<uint32_t>(), perm_.as<uint32_t>(), a, b,
                                                              sa_.as<uint32_t>(), sb_.as<uint32_t>(),
-                                                             head_.as<uint8_t>(), k);
+                                                             head_.as<uint8_t>(), k, over, big_.as<uint32_t>(),
+                                                             ctl_.as<uint32_t>());
   cuda_check(cudaGetLastError(), "gather");
   ++launches_;
   tb = cub_tmp_.bytes;
@@ -1702,7 +1705,7 @@ void Engine::erase_one(const uint32_t* u, const uint32_t* slot, uint64_t k) {
   const uint32_t ks = (uint32_t)std::max<uint64_t>(std::min<uint64_t>(k, n_), 1);
   launch_pdl(k_apply_delete, grid_for((unsigned long long)ks * 32, kBlock, tuning_.apply_blocks_per_sm), kBlock,
              stream_, view(), key_s_.as<uint32_t>(), sa_.as<uint32_t>(), seg_.as<uint32_t>(), nseg_.as<uint32_t>(), k,
-             ctl_.as<uint32_t>());
+             ctl_.as<uint32_t>(), big_.as<uint32_t>());
   cuda_check(cudaGetLastError(), "apply delete");
   ++launches_;
 }
@@ -1981,7 +1984,7 @@ void Engine::enqueue_delete(const uint32_t* u, const uint32_t* slot, uint64_t k)
   const uint32_t ks = (uint32_t)std::max<uint64_t>(std::min<uint64_t>(k, n_), 1);
   launch_pdl(k_apply_delete, grid_for((unsigned long long)ks * 32, kBlock, tuning_.apply_blocks_per_sm), kBlock,
              stream_, view(), key_s_.as<uint32_t>(), sa_.as<uint32_t>(), seg_.as<uint32_t>(), nseg_.as<uint32_t>(), k,
-             ctl_.as<uint32_t>());
+             ctl_.as<uint32_t>(), big_.as<uint32_t>());
   cuda_check(cudaGetLastError(), "apply delete");
   ++launches_;
 }

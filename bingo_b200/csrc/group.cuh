@@ -47,7 +47,9 @@ inline size_t group_smem_bytes(uint32_t ipt) {
 // < n and b nonzero (inserts). Outputs, for positions g < k in sorted order:
 // key_s[g], perm[g] (batch index), sa[g] = a[perm[g]], sb[g] = b[perm[g]];
 // seg[0..*nseg) the positions where a new vertex starts. ctl[0..4) is zeroed
-// and then gets the batch's validation bits (also OR-ed into err).
+// and then gets the batch's validation bits (also OR-ed into err). over > 0:
+// the positions of segments longer than that are listed in big[0..ctl[1]), in
+// no particular order (over < kGroupThreads).
 // Launch: a cluster of CTAS CTAs x kGroupThreads, group_smem_bytes(ipt)
 // dynamic shared memory, ipt = group_ipt(k, CTAS) <= IPT_MAX.
 template <int CTAS, int IPT_MAX>
@@ -55,7 +57,8 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
     k_group_small(const uint32_t* __restrict__ key, const uint32_t* __restrict__ a, const uint32_t* __restrict__ b,
                   uint32_t k, uint32_t n, int end_bit, uint32_t ipt, int check_payload, uint32_t* __restrict__ key_s,
                   uint32_t* __restrict__ perm, uint32_t* __restrict__ sa, uint32_t* __restrict__ sb,
-                  uint32_t* __restrict__ seg, uint32_t* __restrict__ nseg, uint32_t* ctl, uint32_t* err) {
+                  uint32_t* __restrict__ seg, uint32_t* __restrict__ nseg, uint32_t* ctl, uint32_t* err, uint32_t over,
+                  uint32_t* __restrict__ big) {
   namespace cg = cooperative_groups;
   constexpr int BINS = kGroupBins, BITS = kGroupDigitBits;
   static_assert(BINS == kGroupThreads, "one thread per digit in the digit scans");
@@ -270,7 +273,14 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
           if (check_payload && bv[i] == 0u) bits |= E_ZERO_WEIGHT;
         }
         if (v[i].x >= n || (check_payload && av[i] >= n)) bits |= E_RANGE;
-        if (h) seg[cb + wc[i * 32 + w] + __popc(bal & below)] = g;
+        if (h) {
+          seg[cb + wc[i * 32 + w] + __popc(bal & below)] = g;
+          if (over && g + over < k) {  // sorted: longer iff the key that far on is the same (at most a chunk on)
+            const uint32_t j = i * kGroupThreads + t + over;
+            const uint32_t far = j < chunk ? in[j].x : cluster.map_shared_rank(in, c + 1)[j - chunk].x;
+            if (far == v[i].x) big[atomicAdd(ctl + 1, 1u)] = g;
+          }
+        }
       }
     }
   }
