@@ -104,10 +104,12 @@ __global__ void k_validate(const uint32_t* a, const uint32_t* b, const uint32_t*
 
 // Sorted order -> payload columns in sorted order + segment heads.
 // `over` > 0: the positions of segments longer than that are listed in
-// big[0..ctl[1]), in no particular order.
+// big[0..ctl[1]), in no particular order. Ids >= n are not in order (the sort
+// looks at the bits of ids below n), so a batch with such ids, which is
+// refused, can have any number of heads: entries past n are dropped.
 __global__ void k_gather(const uint32_t* key, const uint32_t* perm, const uint32_t* a, const uint32_t* b,
-                         uint32_t* sa, uint32_t* sb, uint8_t* head, unsigned long long k, uint32_t over,
-                         uint32_t* big, uint32_t* ctl) {
+                         uint32_t* sa, uint32_t* sb, uint8_t* head, unsigned long long k, uint32_t n,
+                         uint32_t over, uint32_t* big, uint32_t* ctl) {
   for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < k;
        i += (unsigned long long)gridDim.x * blockDim.x) {
     const uint32_t p = perm[i];
@@ -115,7 +117,10 @@ __global__ void k_gather(const uint32_t* key, const uint32_t* perm, const uint32
     if (b) sb[i] = b[p];
     const bool h = i == 0 || key[i] != key[i - 1];
     head[i] = h;
-    if (h && over && i + over < k && key[i + over] == key[i]) big[atomicAdd(ctl + 1, 1u)] = (uint32_t)i;
+    if (h && over && i + over < k && key[i + over] == key[i]) {
+      const uint32_t at = atomicAdd(ctl + 1, 1u);
+      if (at < n) big[at] = (uint32_t)i;
+    }
   }
 }
 
@@ -1226,7 +1231,7 @@ void Engine::group_by_vertex(const uint32_t* key, const uint32_t* a, const uint3
              "radix sort");
   k_gather<<<grid_for(k, kBlock, 16), kBlock, 0, stream_>>>(key_s_.as<uint32_t>(), perm_.as<uint32_t>(), a, b,
                                                              sa_.as<uint32_t>(), sb_.as<uint32_t>(),
-                                                             head_.as<uint8_t>(), k, over, big_.as<uint32_t>(),
+                                                             head_.as<uint8_t>(), k, n_, over, big_.as<uint32_t>(),
                                                              ctl_.as<uint32_t>());
   cuda_check(cudaGetLastError(), "gather");
   ++launches_;

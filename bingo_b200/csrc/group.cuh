@@ -49,7 +49,9 @@ inline size_t group_smem_bytes(uint32_t ipt) {
 // seg[0..*nseg) the positions where a new vertex starts. ctl[0..4) is zeroed
 // and then gets the batch's validation bits (also OR-ed into err). over > 0:
 // the positions of segments longer than that are listed in big[0..ctl[1]), in
-// no particular order (over < kGroupThreads).
+// no particular order (over < kGroupThreads); big holds min(k, n) entries, as
+// many as a valid batch can have (ids >= n are not in order and can make more
+// heads: theirs are dropped, and so is the batch).
 // Launch: a cluster of CTAS CTAs x kGroupThreads, group_smem_bytes(ipt)
 // dynamic shared memory, ipt = group_ipt(k, CTAS) <= IPT_MAX.
 template <int CTAS, int IPT_MAX>
@@ -278,7 +280,10 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
           if (over && g + over < k) {  // sorted: longer iff the key that far on is the same (at most a chunk on)
             const uint32_t j = i * kGroupThreads + t + over;
             const uint32_t far = j < chunk ? in[j].x : cluster.map_shared_rank(in, c + 1)[j - chunk].x;
-            if (far == v[i].x) big[atomicAdd(ctl + 1, 1u)] = g;
+            if (far == v[i].x) {
+              const uint32_t at = atomicAdd(ctl + 1, 1u);
+              if (at < n) big[at] = g;
+            }
           }
         }
       }
