@@ -350,12 +350,12 @@ void Engine::check_store(bingo_check_report* out) {
   read_tops();
   CheckTotals zero{};
   zero.first_bad = 0xffffffffu;
-  check_buf_.ensure(sizeof(CheckTotals), "store check");
+  reserve(check_buf_, sizeof(CheckTotals), "store check");
   // A sound store's vertices with more than kBigMembers members each own
   // that many entries of the used member arena, so this many list entries
   // suffice; a corrupt store that needs more is checked in place.
   const uint32_t big_cap = (uint32_t)std::min<unsigned long long>(n_, h_top_[A_MEMBER] / kBigMembers + 1);
-  check_big_.ensure((size_t)big_cap * sizeof(BigVertex), "store check");
+  reserve(check_big_, (size_t)big_cap * sizeof(BigVertex), "store check");
   cuda_check(cudaMemcpyAsync(check_buf_.p, &zero, sizeof zero, cudaMemcpyHostToDevice, stream_), "store check");
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_check, kCheckBlock, 0) != cudaSuccess || per_sm <= 0) {

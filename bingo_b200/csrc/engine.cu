@@ -1110,7 +1110,9 @@ void Engine::ensure_batch_scratch(uint64_t k) {
     cuda_check(cudaEventSynchronize(slots_ev_), "slot copy");
     slots_busy_ = false;
   }
-  for (const Scratch& q : batch_scratch(k)) q.buf->ensure(q.bytes, "scratch");
+  scratch_kept_ = false;
+  if (iota_.bytes < kk * 4) iota_n_ = 0;  // allocated anew below (or not, when the device is full)
+  for (const Scratch& q : batch_scratch(k)) reserve(*q.buf, q.bytes, "scratch");
   if (iota_n_ < kk) fill_iota(kk);
   group_cluster_ok();  // probed here, outside any stream capture
 }
@@ -1120,7 +1122,7 @@ void Engine::ensure_batch_scratch(uint64_t k) {
 WalkQueue* Engine::walk_queue(DevBuf& buf, size_t slots) {
   const size_t want = slots * sizeof(WalkQueue);
   if (!buf.p || buf.bytes < want) {
-    buf.ensure(want, "walk queue");
+    reserve(buf, want, "walk queue");
     cuda_check(cudaMemsetAsync(buf.p, 0, buf.bytes, stream_), "walk queue");
   }
   return buf.as<WalkQueue>();
@@ -1253,22 +1255,13 @@ void Engine::grow_arena(int a, unsigned long long min_cap) {
   if (nc < min_cap)
     throw Error(BINGO_ERR_CAPACITY, std::string(kArenaName[a]) + " arena would exceed its 32-bit index range");
   const unsigned long long used = h_top_[a];
-  auto reserve = [&](DevBuf& b, size_t bytes) {  // the kept load scratch makes room when there is none
-    try {
-      b.ensure(bytes, "grow arena");
-    } catch (const Error& e) {
-      if (e.status != BINGO_ERR_CAPACITY || load_slab_in_use_ || !load_slab_.p) throw;
-      load_slab_.release();
-      b.ensure(bytes, "grow arena");
-    }
-  };
   DevBuf fresh;
-  reserve(fresh, nc * kUnitBytes[a]);
+  reserve(fresh, nc * kUnitBytes[a], "grow arena");
   if (used) cuda_check(cudaMemcpyAsync(fresh.p, arena_[a].p, used * kUnitBytes[a], cudaMemcpyDeviceToDevice, stream_),
                        "grow arena copy");
   if (a == A_MEMBER) {
     DevBuf fgs;
-    reserve(fgs, nc * 4);
+    reserve(fgs, nc * 4, "grow arena");
     if (used) cuda_check(cudaMemcpyAsync(fgs.p, gs_.p, used * 4, cudaMemcpyDeviceToDevice, stream_), "grow copy");
     cuda_check(cudaStreamSynchronize(stream_), "grow arena");
     gs_.release();
@@ -1281,6 +1274,40 @@ void Engine::grow_arena(int a, unsigned long long min_cap) {
   fresh.p = nullptr;
   cap_[a] = nc;
   ++arena_gen_;
+}
+
+// All allocations of a handle that may be large: when the device has no room,
+// what is held only to save a later call's allocations makes room first.
+void Engine::reserve(DevBuf& b, size_t want, const char* what) {
+  try {
+    b.ensure(want, what);
+  } catch (const Error& e) {
+    if (e.status != BINGO_ERR_CAPACITY || !give_back()) throw;
+    b.ensure(want, what);
+  }
+}
+
+// Frees what loads keep for the next one, and update scratch that a load left
+// in place; false when there was nothing.
+bool Engine::give_back() {
+  bool any = false;
+  auto drop = [&](DevBuf& b) {
+    any |= b.p != nullptr;
+    b.release();
+  };
+  if (load_slab_in_use_) {  // a load is running in the slab: the updates' own scratch lies beside it
+    for (DevBuf& b : load_own_) drop(b);
+    load_own_iota_ = 0;
+  } else {
+    drop(load_slab_);
+    if (scratch_kept_) {
+      for (const Scratch& q : batch_scratch(1)) drop(*q.buf);
+      iota_n_ = 0;
+      scratch_kept_ = false;
+    }
+  }
+  if (fw_kept_) drop(fw_in_), drop(fw_fixed_);
+  return any;
 }
 
 void Engine::drop_arenas() {
@@ -1298,12 +1325,13 @@ namespace {
 // Whether a buffer kept from the graph before serves for `want` bytes: large
 // enough, and not so large that it holds memory others could use.
 bool fits(const DevBuf& b, size_t want) { return b.p && b.bytes >= want && b.bytes <= 2 * want + (1u << 20); }
-void refit(DevBuf& b, size_t want, const char* what) {
+}  // namespace
+
+void Engine::refit(DevBuf& b, size_t want, const char* what) {
   if (fits(b, want)) return;
   b.release();
-  b.ensure(want, what);
+  reserve(b, want, what);
 }
-}  // namespace
 
 // Arenas for a new graph. Those of the graph before are kept where they fit
 // (allocating and freeing them took most of a load: 18 of 27 ms for R-MAT
@@ -1314,7 +1342,6 @@ void Engine::alloc_arenas(const unsigned long long need[kArenas]) {
   } catch (const Error& e) {
     if (e.status != BINGO_ERR_CAPACITY) throw;
     drop_arenas();
-    if (!load_slab_in_use_) load_slab_.release();
     size_arenas(need);
   }
   cuda_check(cudaMemsetAsync(d_top_, 0, kArenas * sizeof(unsigned long long), stream_), "reset tops");
@@ -1480,11 +1507,10 @@ void Engine::load(const uint32_t* src, const uint32_t* dst, const uint32_t* w, u
   } catch (const Error& e) {
     if (e.status != BINGO_ERR_CAPACITY) throw;
     drop_arenas();
-    load_slab_.release();
     vrec_.release(), meta_.release(), gdesc_.release();
-    vrec_.ensure((size_t)n * sizeof(VertexRec), "vertex records");
-    meta_.ensure((size_t)n * sizeof(VertexMeta), "vertex metadata");
-    gdesc_.ensure((size_t)n * kBits * sizeof(GroupDesc), "group descriptors");
+    reserve(vrec_, (size_t)n * sizeof(VertexRec), "vertex records");
+    reserve(meta_, (size_t)n * sizeof(VertexMeta), "vertex metadata");
+    reserve(gdesc_, (size_t)n * kBits * sizeof(GroupDesc), "group descriptors");
   }
   cuda_check(cudaMemsetAsync(vrec_.p, 0, (size_t)n * sizeof(VertexRec), stream_), "memset");
   cuda_check(cudaMemsetAsync(meta_.p, 0, (size_t)n * sizeof(VertexMeta), stream_), "memset");
@@ -1522,17 +1548,18 @@ void Engine::load_batch(const uint32_t* src, const uint32_t* dst, const uint32_t
     drop_arenas();
     for (const Scratch& q : need) q.buf->release();
     iota_n_ = 0;
-    load_slab_.ensure(total, "scratch");
+    reserve(load_slab_, total, "scratch");
   }
+  scratch_kept_ = false;
   struct Borrow {  // the batch buffers point into the slab while this lives
     Engine& e;
     const std::vector<Scratch>& need;
-    std::vector<DevBuf> own;
-    uint64_t iota_n;
-    Borrow(Engine& e_, const std::vector<Scratch>& need_) : e(e_), need(need_), iota_n(e_.iota_n_) {
+    Borrow(Engine& e_, const std::vector<Scratch>& need_) : e(e_), need(need_) {
       char* p = e.load_slab_.as<char>();
+      e.load_own_.clear();
+      e.load_own_iota_ = e.iota_n_;
       for (const Scratch& q : need) {
-        own.push_back(*q.buf);
+        e.load_own_.push_back(*q.buf);
         q.buf->p = p, q.buf->bytes = q.bytes;
         p += (q.bytes + 255) & ~(size_t)255;
       }
@@ -1540,8 +1567,8 @@ void Engine::load_batch(const uint32_t* src, const uint32_t* dst, const uint32_t
     }
     ~Borrow() {
       cudaStreamSynchronize(e.stream_);  // also after an error: nothing uses the slab past this
-      for (size_t i = 0; i < need.size(); ++i) *need[i].buf = own[i];
-      e.iota_n_ = iota_n;
+      for (size_t i = 0; i < need.size(); ++i) *need[i].buf = e.load_own_[i];
+      e.iota_n_ = e.load_own_iota_;
       e.load_slab_in_use_ = false;
     }
   };
@@ -1566,6 +1593,7 @@ void Engine::load_batch(const uint32_t* src, const uint32_t* dst, const uint32_t
     for (const Scratch& q : need) q.buf->release();
     iota_n_ = 0;
   }
+  scratch_kept_ = true;
 }
 
 void Engine::insert(const uint32_t* src, const uint32_t* dst, const uint32_t* w, uint64_t k, uint32_t* out_slots) {
@@ -1598,12 +1626,13 @@ const uint32_t* Engine::fixed_weights(const float* w, uint64_t k) {
     throw Error(BINGO_ERR_INVALID_ARGUMENT, "float weights need a handle created with weight_mode = BINGO_WEIGHTS_F32");
   if (!w) throw Error(BINGO_ERR_INVALID_ARGUMENT, "null weight array");
   const float* dw = w;
+  fw_kept_ = false;
   if (!is_device_ptr(w)) {
-    fw_in_.ensure(k * 4, "float weights");
+    reserve(fw_in_, k * 4, "float weights");
     cuda_check(cudaMemcpyAsync(fw_in_.p, w, k * 4, cudaMemcpyHostToDevice, stream_), "stage float weights");
     dw = fw_in_.as<float>();
   }
-  fw_fixed_.ensure(k * 4, "float weights");
+  reserve(fw_fixed_, k * 4, "float weights");
   ctl_.ensure(16, "scratch");
   cuda_check(cudaMemsetAsync(ctl_.p, 0, 4, stream_), "ctl");
   k_fixed16<<<grid_for(k, kBlock, 16), kBlock, 0, stream_>>>(dw, k, fw_fixed_.as<uint32_t>(), ctl_.as<uint32_t>());
@@ -1622,6 +1651,7 @@ void Engine::load_f32(const uint32_t* src, const uint32_t* dst, const float* w, 
   const uint32_t* q = m ? fixed_weights(w, m) : nullptr;
   load(src, dst, m ? q : nullptr, m, n);
   // Kept for the next load like the scratch slab, while small.
+  fw_kept_ = true;
   if (fw_in_.bytes + fw_fixed_.bytes > std::max<size_t>(load_slab_.bytes / 4, 64u << 20)) fw_in_.release(), fw_fixed_.release();
 }
 
@@ -1740,13 +1770,13 @@ void Engine::erase_pairs(const uint32_t* u, const uint32_t* v, uint64_t k) {
 // Scratch for translating k pairs (sized before a program is captured).
 void Engine::ensure_pair_scratch(uint64_t k) {
   const uint64_t kk = std::max<uint64_t>(k, 1);
-  pair_key_.ensure(kk * 8, "scratch");
-  pair_key_s_.ensure(kk * 8, "scratch");
-  pair_slot_.ensure(kk * 4, "scratch");
+  reserve(pair_key_, kk * 8, "scratch");
+  reserve(pair_key_s_, kk * 8, "scratch");
+  reserve(pair_slot_, kk * 4, "scratch");
   size_t t_sort = 0;
   cub::DeviceRadixSort::SortPairs(nullptr, t_sort, (const unsigned long long*)nullptr, (unsigned long long*)nullptr,
                                   (const uint32_t*)nullptr, (uint32_t*)nullptr, (int)kk, 0, 64, stream_);
-  cub_tmp_.ensure(t_sort, "scratch");
+  reserve(cub_tmp_, t_sort, "scratch");
 }
 
 // Device arrays u, v -> pair_slot_ (stream-ordered, no host synchronisation):
@@ -1818,7 +1848,7 @@ void Engine::walk(const bingo_walk_job* jobs, uint32_t n_jobs, uint32_t mode) {
   // Staging grows to the next power of two, so a stream of queries of
   // varying size reallocates (a device-wide synchronising cudaFree plus a
   // cudaMalloc) only a few times.
-  if (s_total) wstart_.ensure(pow2_bytes(s_total * 4), "walk staging");
+  if (s_total) reserve(wstart_, pow2_bytes(s_total * 4), "walk staging");
   // Host-bound outputs go through the next staging buffer; its previous
   // copy-out must finish before these kernels overwrite it (a device-side
   // wait, no host synchronisation).
@@ -1832,7 +1862,7 @@ void Engine::walk(const bingo_walk_job* jobs, uint32_t n_jobs, uint32_t mode) {
       else
         cuda_check(cudaStreamWaitEvent(stream_, copy_ev_[ring], 0), "staging reuse");
     }
-    wout_[ring].ensure(pow2_bytes(o_total * 4), "walk staging");
+    reserve(wout_[ring], pow2_bytes(o_total * 4), "walk staging");
     wout = wout_[ring].as<int32_t>();
   }
   for (uint32_t j = 0; j < n_jobs; ++j) {
@@ -1877,8 +1907,8 @@ void Engine::walk(const bingo_walk_job* jobs, uint32_t n_jobs, uint32_t mode) {
     std::vector<uint32_t> pf;
     std::vector<WalkGroup> groups;
     build_walk_groups(dj.data(), n_jobs, tuning_.walk_split != 0, tuning_.walk_order != 0, table, pf, groups);
-    jobs_.ensure(table.size() * sizeof(WalkJobDev), "walk jobs");
-    prefix_.ensure(pf.size() * 4, "walk jobs");
+    reserve(jobs_, table.size() * sizeof(WalkJobDev), "walk jobs");
+    reserve(prefix_, pf.size() * 4, "walk jobs");
     cuda_check(cudaMemcpyAsync(jobs_.p, table.data(), table.size() * sizeof(WalkJobDev), cudaMemcpyHostToDevice,
                                stream_),
                "jobs H2D");
@@ -2105,8 +2135,8 @@ void Engine::run(const bingo_op* ops, uint32_t n_ops, uint32_t flags) {
   if (!table.empty()) {
     const size_t jb = table.size() * sizeof(WalkJobDev), pb = pf.size() * 4, qb = groups.size() * sizeof(WalkQueue);
     if (jb > prog_jobs_.bytes || pb > prog_prefix_.bytes || qb > prog_queue_.bytes) drop_graph();
-    prog_jobs_.ensure(jb, "program jobs");
-    prog_prefix_.ensure(pb, "program jobs");
+    reserve(prog_jobs_, jb, "program jobs");
+    reserve(prog_prefix_, pb, "program jobs");
     walk_queue(prog_queue_, groups.size());
     cuda_check(cudaMemcpyAsync(prog_jobs_.p, table.data(), jb, cudaMemcpyHostToDevice, stream_), "program jobs H2D");
     cuda_check(cudaMemcpyAsync(prog_prefix_.p, pf.data(), pb, cudaMemcpyHostToDevice, stream_), "program jobs H2D");
@@ -2296,8 +2326,8 @@ void Engine::philox_batch(const uint32_t* ctr4, uint64_t count, uint64_t key, ui
   if (!count) return;
   if (!ctr4 || !out4) throw Error(BINGO_ERR_INVALID_ARGUMENT, "null array");
   DevBuf c, o;
-  c.ensure(count * 16, "philox");
-  o.ensure(count * 16, "philox");
+  reserve(c, count * 16, "philox");
+  reserve(o, count * 16, "philox");
   cuda_check(cudaMemcpyAsync(c.p, ctr4, count * 16, cudaMemcpyDefault, stream_), "philox H2D");
   k_philox<<<grid_for(count, kBlock), kBlock, 0, stream_>>>(c.as<uint32_t>(), count, (uint32_t)key,
                                                            (uint32_t)(key >> 32), o.as<uint32_t>());
@@ -2479,11 +2509,11 @@ bool Engine::save_state(StateCopy& c) {
   cuda_check(cudaStreamSynchronize(stream_), "state copy");
   read_tops();
   try {
-    c.vrec.ensure((size_t)n_ * sizeof(VertexRec), "state copy");
-    c.meta.ensure((size_t)n_ * sizeof(VertexMeta), "state copy");
-    c.gdesc.ensure((size_t)n_ * kBits * sizeof(GroupDesc), "state copy");
-    for (int a = 0; a < kArenas; ++a) c.arena[a].ensure(std::max(1ull, h_top_[a]) * kUnitBytes[a], "state copy");
-    c.gs.ensure(std::max(1ull, h_top_[A_MEMBER]) * 4, "state copy");
+    reserve(c.vrec, (size_t)n_ * sizeof(VertexRec), "state copy");
+    reserve(c.meta, (size_t)n_ * sizeof(VertexMeta), "state copy");
+    reserve(c.gdesc, (size_t)n_ * kBits * sizeof(GroupDesc), "state copy");
+    for (int a = 0; a < kArenas; ++a) reserve(c.arena[a], std::max(1ull, h_top_[a]) * kUnitBytes[a], "state copy");
+    reserve(c.gs, std::max(1ull, h_top_[A_MEMBER]) * 4, "state copy");
   } catch (const Error&) {
     cudaGetLastError();
     c.release();
@@ -2699,9 +2729,9 @@ void Engine::restore(const char* path) {
   ++arena_gen_;
   n_ = H.n;
   vrec_.release(), meta_.release(), gdesc_.release();
-  vrec_.ensure((size_t)n_ * sizeof(VertexRec), "vertex records");
-  meta_.ensure((size_t)n_ * sizeof(VertexMeta), "vertex metadata");
-  gdesc_.ensure((size_t)n_ * kBits * sizeof(GroupDesc), "group descriptors");
+  reserve(vrec_, (size_t)n_ * sizeof(VertexRec), "vertex records");
+  reserve(meta_, (size_t)n_ * sizeof(VertexMeta), "vertex metadata");
+  reserve(gdesc_, (size_t)n_ * kBits * sizeof(GroupDesc), "group descriptors");
   const unsigned long long need[kArenas] = {H.top[0], H.top[1], H.top[2], H.top[3], H.top[4]};
   alloc_arenas(need);
   struct Part {

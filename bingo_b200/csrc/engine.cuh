@@ -112,6 +112,7 @@ class Engine {
   WalkJobDev make_job(const bingo_walk_job& J) const;
   void check_walk_job(const bingo_walk_job& J) const;
   void prepare_batches(uint64_t k) { ensure_batch_scratch(k); }
+  void reserve(DevBuf& b, size_t want, const char* what);
   // The serving scheduler enqueues update batches without a host wait per
   // call (it polls an event instead); device-reported errors then surface
   // through sync().
@@ -155,6 +156,9 @@ class Engine {
       slots_, cub_tmp_;
   DevBuf load_slab_;                          // a load's scratch, kept for the next one
   bool load_slab_in_use_ = false;
+  std::vector<DevBuf> load_own_;              // the batch buffers' own memory while a load runs in the slab
+  uint64_t load_own_iota_ = 0;
+  bool scratch_kept_ = false, fw_kept_ = false;  // scratch, float buffers: held since a load, not in use since
   DevBuf pair_key_, pair_key_s_, pair_slot_;  // delete-by-pair translation
   DevBuf fw_in_, fw_fixed_;                   // float weights: staged input, 16.16 fixed point
   DevBuf check_buf_, check_big_;              // store check: totals, large-vertex list
@@ -190,6 +194,8 @@ class Engine {
   void ensure_batch_scratch(uint64_t k);
   void fill_iota(uint64_t k);
   void load_batch(const uint32_t* src, const uint32_t* dst, const uint32_t* w, uint64_t m);
+  bool give_back();
+  void refit(DevBuf& b, size_t want, const char* what);
   void drop_arenas();
   void drop_store();
   void size_arenas(const unsigned long long need[kArenas]);

@@ -234,14 +234,14 @@ Server::Server(Engine& eng, const bingo_serve_config& cfg) : eng_(eng), cfg_(cfg
              "serve completion words");
   std::memset((void*)done_seq_, 0, (kServeMaxJobs + 1) * sizeof(unsigned long long));
   cuda_check(cudaHostGetDevicePointer((void**)&d_done_seq_, (void*)done_seq_, 0), "serve completion words");
-  ctlbuf_.ensure(sizeof(ServeCtl), "serve control block");
+  eng_.reserve(ctlbuf_, sizeof(ServeCtl), "serve control block");
   d_ctl_ = ctlbuf_.as<ServeCtl>();
   std::memset(&ctl_, 0, sizeof ctl_);
   cuda_check(cudaMemcpy(d_ctl_, &ctl_, sizeof ctl_, cudaMemcpyHostToDevice), "serve control block");
-  jobs_.ensure(kServeMaxJobs * sizeof(WalkJobDev), "serve job ring");
-  state_.ensure(sizeof(ServeDevState), "serve state");
+  eng_.reserve(jobs_, kServeMaxJobs * sizeof(WalkJobDev), "serve job ring");
+  eng_.reserve(state_, sizeof(ServeDevState), "serve state");
   cuda_check(cudaMemset(state_.p, 0, sizeof(ServeDevState)), "serve state");
-  budget_.ensure(cfg_.output_budget_bytes, "serve output budget");
+  eng_.reserve(budget_, cfg_.output_budget_bytes, "serve output budget");
   eng_.prepare_batches(cfg_.max_update_batch);
   cuda_check(cudaEventCreateWithFlags(&upd_ev_, cudaEventDisableTiming), "serve update event");
   thread_ = std::thread([this] { loop(); });
