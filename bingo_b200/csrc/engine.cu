@@ -1323,8 +1323,10 @@ void Engine::drop_store() {
 
 namespace {
 // Whether a buffer kept from the graph before serves for `want` bytes: large
-// enough, and not so large that it holds memory others could use.
-bool fits(const DevBuf& b, size_t want) { return b.p && b.bytes >= want && b.bytes <= 2 * want + (1u << 20); }
+// enough, and at most a sixteenth larger. Loads of the same graph again, or of
+// one that has changed a little, keep all of theirs; nothing could use what a
+// larger buffer holds past its capacity, not even this handle.
+bool fits(const DevBuf& b, size_t want) { return b.p && b.bytes >= want && b.bytes <= want + want / 16 + (1u << 20); }
 }  // namespace
 
 void Engine::refit(DevBuf& b, size_t want, const char* what) {
