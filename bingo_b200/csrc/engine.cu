@@ -24,6 +24,7 @@
 
 #include "engine.cuh"
 #include "group.cuh"
+#include "near.h"
 #include "serve.cuh"
 #include "store.cuh"
 #include "walk.cuh"
@@ -484,9 +485,11 @@ __global__ void __launch_bounds__(kBlock, 3) k_apply_delete(const __grid_constan
       prefetch_l2(S.gdesc + (size_t)u * kBits + kBits / 2);
       prefetch_l2(S.vrec + u);
       if (slot < M->ecnt) {
-        const uint32_t ebp = S.edges[M->eoff + slot].ebp;
-        prefetch_l2(S.bp + M->bpoff + ebp);
-        prefetch_l2(S.bp + M->bpoff + ebp + 7);
+        const EdgeRec e = S.edges[M->eoff + slot];
+        if (e.w) {
+          prefetch_l2(S.bp + M->bpoff + e.ebp);
+          prefetch_l2(S.bp + M->bpoff + e.ebp + near_last(e.w));
+        }
       }
     }
     for (uint32_t todo = __ballot_sync(kFull, u < S.n && e - b <= kBigDelete); todo; todo &= todo - 1) {
