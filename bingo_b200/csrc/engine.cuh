@@ -13,6 +13,7 @@
 #include "../../include/bingo.h"
 #include "claim.h"
 #include "common.cuh"
+#include "tune_search.h"
 #include "walk.cuh"
 
 namespace bingo {
@@ -48,16 +49,6 @@ struct DevBuf {
 };
 
 class Server;
-
-// Launch and batching knobs (bingo_tuning); none changes any result.
-struct Tuning {
-  uint32_t walk_chunk = 0;          // 0 = each walk kernel's default (walk_default_chunk)
-  uint32_t walk_blocks_per_sm = 0;  // 0 = each walk kernel's default (walk_default_bps)
-  uint32_t walk_split = 0;
-  uint32_t walk_order = 1;
-  uint32_t update_chunk = 0;  // 0 = whole batch
-  uint32_t apply_blocks_per_sm = 8;
-};
 
 // A device copy of the graph store (the update knobs are timed on the live
 // graph and undone from it).

@@ -7,28 +7,13 @@
 // then restoring the store from a device copy taken before the first trial,
 // so the graph is the same when the call returns.
 //
-// Search: one coordinate pass in a fixed order (walk_chunk, walk_split,
-// walk_order, walk_blocks_per_sm, a second look at walk_chunk around the
-// pick, then update_chunk and apply_blocks_per_sm). A candidate replaces the
-// current choice only when its median wall time is at least 1 % lower, so
-// noise does not move the knobs.
+// Search: tune_search.h.
 #include <algorithm>
 #include <chrono>
-#include <vector>
 
 #include "engine.cuh"
 
 namespace bingo {
-
-namespace {
-
-double median(std::vector<double> v) {
-  std::sort(v.begin(), v.end());
-  const size_t m = v.size() / 2;
-  return v.size() % 2 ? v[m] : 0.5 * (v[m - 1] + v[m]);
-}
-
-}  // namespace
 
 void Engine::autotune(const bingo_tune_request& R, bingo_tune_report* out) {
   const NvtxRange nvtx_("bingo autotune");
@@ -52,37 +37,16 @@ void Engine::autotune(const bingo_tune_request& R, bingo_tune_report* out) {
 
   double walk_start = -1, walk_best = -1;
   if (R.n_jobs) {
-    auto time_walks = [&](const Tuning& t) {
+    auto once = [&](const Tuning& t) {
       tuning_ = t;
-      std::vector<double> v;
-      for (int r = 0; r <= reps; ++r) {
-        const double ms = wall_ms([&] { walk(R.jobs, R.n_jobs, BINGO_WALK_BATCHED); });
-        if (r) v.push_back(ms);  // the first run warms up
-      }
-      ++cand;
-      return median(v);
-    };
-    auto try_knob = [&](uint32_t Tuning::*f, const std::vector<uint32_t>& vals) {
-      for (uint32_t x : vals) {
-        if (best.*f == x) continue;
-        Tuning t = best;
-        t.*f = x;
-        const double ms = time_walks(t);
-        if (ms < walk_best * 0.99) walk_best = ms, best = t;
-      }
+      return wall_ms([&] { walk(R.jobs, R.n_jobs, BINGO_WALK_BATCHED); });
     };
     try {
-      walk_start = walk_best = time_walks(best);
-      try_knob(&Tuning::walk_chunk, {8, 16, 32, 64, 128, 256});
+      KnobSearch<decltype(once)> s(best, reps, once);
       bool mixed = false;
       for (uint32_t j = 1; j < R.n_jobs; ++j) mixed |= R.jobs[j].app != R.jobs[0].app;
-      if (mixed) try_knob(&Tuning::walk_split, {0, 1});
-      if (R.n_jobs > 1) try_knob(&Tuning::walk_order, {1, 0});
-      try_knob(&Tuning::walk_blocks_per_sm, {0, 6, 4, 3, 2});
-      std::vector<uint32_t> around;  // 0 (each kernel's default) has no neighbours
-      if (best.walk_chunk > 1) around.push_back(best.walk_chunk / 2);
-      if (best.walk_chunk && best.walk_chunk < 1024) around.push_back(best.walk_chunk * 2);
-      try_knob(&Tuning::walk_chunk, around);
+      search_walk_knobs(s, R.n_jobs > 1, mixed);
+      best = s.best, walk_start = s.ms_start, walk_best = s.ms_best, cand += s.candidates;
     } catch (...) {
       tuning_ = start;
       throw;
@@ -95,36 +59,18 @@ void Engine::autotune(const bingo_tune_request& R, bingo_tune_report* out) {
       throw Error(BINGO_ERR_INVALID_ARGUMENT, "null update array");
     StateCopy snap;
     if (save_state(snap)) {
-      auto time_updates = [&](const Tuning& t) {
+      auto once = [&](const Tuning& t) {
         tuning_ = t;
-        std::vector<double> v;
-        for (int r = 0; r <= reps; ++r) {
-          restore_state(snap);
-          const double ms = wall_ms([&] {
-            if (R.n_ins) insert(R.ins_src, R.ins_dst, R.ins_w, R.n_ins, nullptr);
-            if (R.n_del) erase(R.del_u, R.del_slot, R.n_del);
-          });
-          if (r) v.push_back(ms);
-        }
-        ++cand;
-        return median(v);
-      };
-      auto try_knob = [&](uint32_t Tuning::*f, const std::vector<uint32_t>& vals) {
-        for (uint32_t x : vals) {
-          if (best.*f == x) continue;
-          Tuning t = best;
-          t.*f = x;
-          const double ms = time_updates(t);
-          if (ms < upd_best * 0.99) upd_best = ms, best = t;
-        }
+        restore_state(snap);
+        return wall_ms([&] {
+          if (R.n_ins) insert(R.ins_src, R.ins_dst, R.ins_w, R.n_ins, nullptr);
+          if (R.n_del) erase(R.del_u, R.del_slot, R.n_del);
+        });
       };
       try {
-        upd_start = upd_best = time_updates(best);
-        const uint64_t kmax = std::max(R.n_ins, R.n_del);
-        std::vector<uint32_t> chunks{0};
-        for (uint64_t c = kmax / 2; c >= 16384 && chunks.size() < 4; c /= 2) chunks.push_back((uint32_t)c);
-        try_knob(&Tuning::update_chunk, chunks);
-        try_knob(&Tuning::apply_blocks_per_sm, {8, 4, 16, 32});
+        KnobSearch<decltype(once)> s(best, reps, once);
+        search_update_knobs(s, std::max(R.n_ins, R.n_del));
+        best = s.best, upd_start = s.ms_start, upd_best = s.ms_best, cand += s.candidates;
         restore_state(snap);
       } catch (...) {
         tuning_ = start;
