@@ -1342,6 +1342,7 @@ void Engine::refit(DevBuf& b, size_t want, const char* what) {
 // (allocating and freeing them took most of a load: 18 of 27 ms for R-MAT
 // 20); when the device has no room beside them they are freed first.
 void Engine::alloc_arenas(const unsigned long long need[kArenas]) {
+  std::memset(h_top_, 0, kArenas * sizeof(unsigned long long));  // nothing to move when an arena grows to its minimum
   try {
     size_arenas(need);
   } catch (const Error& e) {
@@ -1350,7 +1351,6 @@ void Engine::alloc_arenas(const unsigned long long need[kArenas]) {
     size_arenas(need);
   }
   cuda_check(cudaMemsetAsync(d_top_, 0, kArenas * sizeof(unsigned long long), stream_), "reset tops");
-  std::memset(h_top_, 0, kArenas * sizeof(unsigned long long));
   ++arena_gen_;
 }
 
