@@ -570,7 +570,8 @@ __global__ void __launch_bounds__(kBlock) k_pair_slots(StoreView S, const unsign
 
 // Persistent walk kernel with per-lane refill. Each warp owns a range of
 // walk items and hands them to idle lanes; when the range runs out it pulls
-// the next `chunk` items from one device counter (WalkQueue, zero at launch
+// the next `chunk` items (mixed tables with chunk = 0: as many as next_claim
+// says) from one device counter (WalkQueue, zero at launch
 // and zeroed again by the last warp to finish). MULTI = false: every item is
 // a walk of the single job J0.
 // MULTI = true: items index the concatenated jobs of a device job table
@@ -630,6 +631,7 @@ __global__ void __launch_bounds__(kBlock, walk_min_blocks(APP))
   Rand4 ahead{0, 0, 0, 0};
   constexpr int A = APP == APP_SAMPLING ? APP_DEEPWALK : APP;
   bool active = false, drained = false;
+  uint32_t turn = 0, claim = kClaimMin, claimed = 0;  // steps so far; the last claim's size and step
   const uint32_t warps = gridDim.x * (kBlock / 32);
   // A small launch's walks spread over all its warps (walks that take trials
   // spread inside theirs).
@@ -640,10 +642,12 @@ __global__ void __launch_bounds__(kBlock, walk_min_blocks(APP))
     if (idle) room = lanes - min(lanes, 32u - __popc(idle));
     while (idle && room && !drained) {
       if (wb >= we) {
+        const uint32_t c = APP >= 0 || chunk ? chunk : turn ? next_claim(claim, turn - claimed) : kClaimMin;
+        claim = c, claimed = turn;
         unsigned long long base = 0;
-        if (lane == 0) base = min(atomicAdd(&queue->next, (unsigned long long)chunk), (unsigned long long)total);
+        if (lane == 0) base = min(atomicAdd(&queue->next, (unsigned long long)c), (unsigned long long)total);
         base = __shfl_sync(kFull, (uint32_t)base, 0);
-        if (!claim_range(base, total, chunk, &wb, &we)) {
+        if (!claim_range(base, total, c, &wb, &we)) {
           drained = true;
           break;
         }
@@ -672,6 +676,7 @@ __global__ void __launch_bounds__(kBlock, walk_min_blocks(APP))
       continue;
     }
     if (!kRows) continue;
+    ++turn;
     const WalkJobDev& J = MULTI ? jobs[jid] : J0;
     bool out = false, end = false;
     uint32_t pos = 0;
@@ -723,12 +728,13 @@ unsigned walk_blocks_per_sm() {
 // 4 blocks: past that the concurrent random reads only queue (DeepWalk, R-MAT
 // 20, at 4 and 8 blocks: 26.3 and 21.7 G steps/s). Claims: what a warp holds
 // unstarted waits for its lanes, which is worst for long walks: 16 jobs of
-// all apps on R-MAT 20 (1.1 M walks) take 3.3 ms at 32 walks per claim, 2.2
-// at 8 and 1.95 at 4; DeepWalk (1 M walks) 1080 us at 8, 1093 at 16. A launch
-// that fits its lanes claims each warp's share at once. One-hop sampling (one
-// step per item) keeps the occupancy limit and 32.
+// all apps on R-MAT 20 (1.1 M walks) took 3.3 ms at 32 walks per claim, 2.2
+// at 8 and 1.95 at 4; DeepWalk (1 M walks) 1080 us at 8, 1093 at 16; node2vec
+// 4. Mixed tables (0) fit their claims to the walks they meet (next_claim). A
+// launch that fits its lanes claims each warp's share at once. One-hop sampling
+// (one step per item) keeps the occupancy limit and 32.
 constexpr unsigned walk_default_bps(int app) { return app == APP_DEEPWALK || app == APP_PPR ? 4 : 0; }
-constexpr uint32_t walk_default_chunk(int app) { return app == APP_NODE2VEC || app < 0 ? 4 : app == APP_DEEPWALK ? 8 : 32; }
+constexpr uint32_t walk_default_chunk(int app) { return app < 0 ? 0 : app == APP_NODE2VEC ? 4 : app == APP_DEEPWALK ? 8 : 32; }
 
 // Blocks per SM for a walk launch of `app` (-1: mixed table): the tuned or
 // default figure, capped by occupancy.

@@ -390,7 +390,9 @@ typedef struct bingo_tune_report {
 
 /* Coordinate search: walk_chunk, walk_split, walk_order, walk_blocks_per_sm,
  * then update_chunk and apply_blocks_per_sm; a candidate replaces the
- * current choice when its median is at least 1 % lower. */
+ * current choice when its median is at least 1 % lower. The choice is timed
+ * against the starting knobs once more, in turn, and kept only when it is
+ * again at least 1 % faster. */
 int bingo_autotune(bingo_handle* h, const bingo_tune_request* req, bingo_tune_report* out);
 
 /* Scheduler counters since bingo_serve_start (times in ns of scheduler-thread wall time). */
