@@ -576,7 +576,8 @@ __global__ void __launch_bounds__(kBlock) k_pair_slots(StoreView S, const unsign
 // a walk of the single job J0.
 // MULTI = true: items index the concatenated jobs of a device job table
 // (prefix = running walk counts) and each lane follows its own job; APP >= 0
-// when every job of the table has that app, APP < 0 for a mixed table.
+// when every job of the table has that app, APP_MIXED for any jobs, APP_FIRST
+// for any but node2vec.
 // `chunk` (walks per warp refill) is a tuning knob (Tuning::walk_chunk).
 static_assert(kBlock % 32 == 0, "whole warps");
 
@@ -585,12 +586,13 @@ static_assert(kBlock % 32 == 0, "whole warps");
 // at 4 (1 M walks: 1953 us; 2209 at 3); mixed tables, where the longest walks'
 // steps set the time, at 3 (16 jobs: 1716 us; 1833 at 4, 1929 at 2).
 constexpr int walk_min_blocks(int app) {
-  return app == APP_SAMPLING ? 8 : app < 0 ? 3 : 4;
+  return app == APP_SAMPLING ? 8 : app == APP_MIXED ? 3 : 4;
 }
 // Entries of a lane's output line (RowStage): 128 bytes, and 64 where the
 // trial scratch also takes shared memory (L1 holds the reads in flight, so
 // what lines take from it counts: node2vec and mixed tables lose 3 % at 128).
-constexpr int walk_line(int app) { return app == APP_NODE2VEC || app < 0 ? 16 : 32; }
+constexpr bool walk_trials(int app) { return app == APP_NODE2VEC || app == APP_MIXED; }  // steps may take several
+constexpr int walk_line(int app) { return walk_trials(app) ? 16 : 32; }
 
 // The job of a work item: the last one that starts at or before it.
 __device__ __forceinline__ uint32_t job_of_item(const uint32_t* __restrict__ prefix, uint32_t n_jobs, uint32_t item) {
@@ -612,7 +614,7 @@ __global__ void __launch_bounds__(kBlock, walk_min_blocks(APP))
   constexpr int kLine = walk_line(APP);
   using Stage = RowStage<kLine>;
   constexpr bool kRows = APP != APP_SAMPLING;                   // sampling jobs write no rows
-  constexpr bool kTrials = APP == APP_NODE2VEC || APP < 0;       // walks whose steps may take several trials
+  constexpr bool kTrials = walk_trials(APP);
   __shared__ int32_t obuf[kRows ? kBlock * Stage::kPitch : 1];
   __shared__ TrialScratch trials[kTrials ? kBlock / 32 : 1];
   __shared__ WalkJobDev one;  // the single job, where lanes index jobs
@@ -631,7 +633,8 @@ __global__ void __launch_bounds__(kBlock, walk_min_blocks(APP))
   Rand4 ahead{0, 0, 0, 0};
   constexpr int A = APP == APP_SAMPLING ? APP_DEEPWALK : APP;
   bool active = false, drained = false;
-  uint32_t turn = 0, claim = kClaimMin, claimed = 0;  // steps so far; the last claim's size and step
+  // Steps so far; the last claim's size and step; walks claimed.
+  uint32_t turn = 0, claim = kClaimMin, claimed = 0, taken = 0;
   const uint32_t warps = gridDim.x * (kBlock / 32);
   // A small launch's walks spread over all its warps (walks that take trials
   // spread inside theirs).
@@ -642,8 +645,8 @@ __global__ void __launch_bounds__(kBlock, walk_min_blocks(APP))
     if (idle) room = lanes - min(lanes, 32u - __popc(idle));
     while (idle && room && !drained) {
       if (wb >= we) {
-        const uint32_t c = APP >= 0 || chunk ? chunk : turn ? next_claim(claim, turn - claimed) : kClaimMin;
-        claim = c, claimed = turn;
+        const uint32_t c = APP >= 0 || chunk ? chunk : taken >= 32 ? next_claim(claim, turn - claimed) : kClaimMin;
+        claim = c, claimed = turn, taken += c;
         unsigned long long base = 0;
         if (lane == 0) base = min(atomicAdd(&queue->next, (unsigned long long)c), (unsigned long long)total);
         base = __shfl_sync(kFull, (uint32_t)base, 0);
@@ -663,7 +666,7 @@ __global__ void __launch_bounds__(kBlock, walk_min_blocks(APP))
           jid = job_of_item(prefix, n_jobs, item);
           active = walk_begin<APP, kLine, !kTrials>(W, jobs[jid], item - prefix[jid], s, buf, moves);
         }
-        if (A == APP_DEEPWALK && active) {
+        if ((A == APP_DEEPWALK || A == APP_FIRST) && active) {
           const WalkJobDev& J = MULTI ? jobs[jid] : J0;
           ahead = philox(s.i, 1, 0, J.job, J.k0, J.k1);
         }
@@ -733,7 +736,7 @@ unsigned walk_blocks_per_sm() {
 // 4. Mixed tables (0) fit their claims to the walks they meet (next_claim). A
 // launch that fits its lanes claims each warp's share at once. One-hop sampling
 // (one step per item) keeps the occupancy limit and 32.
-constexpr unsigned walk_default_bps(int app) { return app == APP_DEEPWALK || app == APP_PPR ? 4 : 0; }
+constexpr unsigned walk_default_bps(int app) { return app == APP_SAMPLING || walk_trials(app) ? 0 : 4; }
 constexpr uint32_t walk_default_chunk(int app) { return app < 0 ? 0 : app == APP_NODE2VEC ? 4 : app == APP_DEEPWALK ? 8 : 32; }
 
 // Blocks per SM for a walk launch of `app` (-1: mixed table): the tuned or
@@ -745,7 +748,7 @@ unsigned walk_bps(unsigned occ, const Tuning& t, int app) {
 uint32_t walk_chunk_of(const Tuning& t, int app, uint32_t total, unsigned grid) {
   if (t.walk_chunk) return t.walk_chunk;
   const uint32_t warps = grid * (kBlock / 32);
-  const bool one_fill = app != APP_NODE2VEC && app >= 0 && total <= 32ull * warps;  // every warp claims its share at once
+  const bool one_fill = !walk_trials(app) && total <= 32ull * warps;  // every warp claims its share at once
   return one_fill ? walk_share(total, warps) : walk_default_chunk(app);
 }
 
@@ -753,7 +756,7 @@ uint32_t walk_chunk_of(const Tuning& t, int app, uint32_t total, unsigned grid) 
 // walk_per_block walks per block: half-full warps on twice the SMs finish
 // sooner (16,384 DeepWalk walks of 80 on R-MAT 14: 80 us at 256 walks per
 // block, 73 at 128), and walks that take trials use the idle lanes.
-constexpr unsigned walk_per_block(int app) { return app == APP_NODE2VEC || app < 0 ? 64 : app == APP_SAMPLING ? 256 : 128; }
+constexpr unsigned walk_per_block(int app) { return walk_trials(app) ? 64 : app == APP_SAMPLING ? 256 : 128; }
 template <int APP, bool MULTI>
 unsigned walk_grid(unsigned long long total, const Tuning& t) {
   return grid_for(total, walk_per_block(APP), walk_bps(walk_blocks_per_sm<APP, MULTI>(), t, APP));
@@ -775,7 +778,8 @@ void launch_walk_table(cudaStream_t st, int app, const WalkView& W, const WalkJo
              : app == APP_NODE2VEC ? launch_walk<APP_NODE2VEC, true>
              : app == APP_PPR      ? launch_walk<APP_PPR, true>
              : app == APP_SAMPLING ? launch_walk<APP_SAMPLING, true>
-                                   : launch_walk<-1, true>;
+             : app == APP_FIRST    ? launch_walk<APP_FIRST, true>
+                                   : launch_walk<APP_MIXED, true>;
   go(st, W, J0, jobs, prefix, n_jobs, total, queue, t);
   cuda_check(cudaGetLastError(), "walk launch");
 }
@@ -812,13 +816,14 @@ void walk_carveouts(int device) {
   if (std::find(done.begin(), done.end(), device) != done.end()) return;
   walk_carveout<APP_DEEPWALK, false>(4), walk_carveout<APP_DEEPWALK, true>(4);
   walk_carveout<APP_PPR, false>(4), walk_carveout<APP_PPR, true>(4);
-  walk_carveout<APP_NODE2VEC, false>(4), walk_carveout<APP_NODE2VEC, true>(4), walk_carveout<-1, true>(3);
+  walk_carveout<APP_NODE2VEC, false>(4), walk_carveout<APP_NODE2VEC, true>(4), walk_carveout<APP_MIXED, true>(3);
+  walk_carveout<APP_FIRST, true>(4);
   done.push_back(device);
 }
 
 // A job table for one persistent launch: jobs of one app (or all apps).
 struct WalkGroup {
-  int app;            // app of every job, or -1 for a mixed table
+  int app;            // app of every job, or APP_MIXED, or APP_FIRST
   size_t job_off;     // first job in the concatenated table
   size_t pf_off;      // first prefix entry (n_jobs + 1 entries)
   uint32_t n_jobs;
@@ -826,6 +831,17 @@ struct WalkGroup {
 };
 
 double walk_cost(const WalkJobDev& J);
+
+// The kernel of a table of any jobs. Without node2vec jobs there is one draw
+// per step and nothing to list: 16 DeepWalk jobs on R-MAT 16 (108,000 walks x
+// 40) take 107 us in the mixed kernel and 78 in this one, 16 PPR jobs 116 and
+// 87, 16 one-hop jobs 29 and 15. (One kernel for all such tables, so that a
+// captured program is kept while its jobs change among these apps.)
+int table_app(const WalkJobDev* in, uint32_t n) {
+  for (uint32_t j = 0; j < n; ++j)
+    if (in[j].app == APP_NODE2VEC && in[j].n) return APP_MIXED;
+  return APP_FIRST;
+}
 
 // Appends the jobs `in` to (table, prefix) as one group per app present
 // (or one mixed group), each ordered by expected walk cost, most expensive
@@ -835,7 +851,7 @@ double walk_cost(const WalkJobDev& J);
 void build_walk_groups(const WalkJobDev* in, uint32_t n, bool split, bool longest_first,
                        std::vector<WalkJobDev>& table, std::vector<uint32_t>& prefix, std::vector<WalkGroup>& groups) {
   std::vector<uint32_t> idx;
-  for (int app = split ? 0 : -1; app <= (split ? 3 : -1); ++app) {
+  for (int app = split ? 0 : APP_MIXED; app <= (split ? 3 : APP_MIXED); ++app) {
     idx.clear();
     for (uint32_t j = 0; j < n; ++j)
       if ((app < 0 || in[j].app == app) && in[j].n) idx.push_back(j);
@@ -843,7 +859,7 @@ void build_walk_groups(const WalkJobDev* in, uint32_t n, bool split, bool longes
     if (longest_first)
       std::stable_sort(idx.begin(), idx.end(),
                        [&](uint32_t a, uint32_t b) { return walk_cost(in[a]) > walk_cost(in[b]); });
-    WalkGroup g{app, table.size(), prefix.size(), (uint32_t)idx.size(), 0};
+    WalkGroup g{app < 0 ? table_app(in, n) : app, table.size(), prefix.size(), (uint32_t)idx.size(), 0};
     uint64_t t = 0;
     prefix.push_back(0);
     for (uint32_t j : idx) {
@@ -2140,6 +2156,7 @@ void Engine::run(const bingo_op* ops, uint32_t n_ops, uint32_t flags) {
     grp_begin[i] = groups.size();
     build_walk_groups(dj.data(), (uint32_t)dj.size(), split, tuning_.walk_order != 0, table, pf, groups);
     grp_end[i] = groups.size();
+    for (size_t gi = grp_begin[i]; gi < grp_end[i]; ++gi) mix((uint64_t)(groups[gi].app + 8));
   }
   // Job tables are read by the walk kernels from device memory, so their
   // contents may change between replays of a captured program.
@@ -2327,7 +2344,7 @@ void Engine::walk_noalloc(const bingo_walk_job* jobs, uint32_t n_jobs) {
   cuda_check(cudaGetLastError(), "no-alloc job staging");
   ++launches_;
   const WalkView W = wview();
-  launch_walk_table(stream_, -1, W, dj[0], scratch->jobs, scratch->prefix, n_jobs, (uint32_t)total, &scratch->queue,
+  launch_walk_table(stream_, table_app(dj, n_jobs), W, dj[0], scratch->jobs, scratch->prefix, n_jobs, (uint32_t)total, &scratch->queue,
                     tuning_);
   ++launches_;
   finish_call();

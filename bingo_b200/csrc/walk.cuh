@@ -19,6 +19,8 @@ constexpr uint32_t kMaxPprSteps = 1u << 20;
 constexpr uint32_t kWalkPprTail = 1u;
 
 enum AppId : int { APP_DEEPWALK = 0, APP_NODE2VEC = 1, APP_PPR = 2, APP_SAMPLING = 3 };
+// Kernels of job tables: jobs of any app, and jobs that are not node2vec.
+constexpr int APP_MIXED = -1, APP_FIRST = -2;
 
 // One walk job as the kernels see it (starts/out are device pointers).
 struct WalkJobDev {
@@ -238,18 +240,23 @@ struct Proposal {
 // after the record's read, 72 under it, 68 so); PPR's two blocks are longer
 // than that read and stay under the record's (100,003 walks: 225 us, 227
 // ahead).
+//
+// APP_FIRST is a table that mixes the first-order apps: its lanes draw as
+// their job's app does, and read together.
 template <int APP>
 __device__ __forceinline__ Proposal walk_propose(const WalkView& W, const WalkJobDev& J, const LaneWalk& s,
                                                  Rand4& ahead) {
   Proposal p{-1, true, false, 0, 0};
-  if (APP == APP_PPR) {
-    Rand4 r = philox(s.i, s.j, 0, J.job, J.k0, J.k1);
+  const bool ppr = APP == APP_PPR || (APP == APP_FIRST && J.app == APP_PPR);
+  Rand4 r = ahead;
+  if (ppr) {
+    r = philox(s.i, s.j, 0, J.job, J.k0, J.k1);
     uint32_t ax = philox(s.i, s.j, 1, J.job, J.k0, J.k1).x;
     asm volatile("" : "+r"(r.x), "+r"(r.y), "+r"(r.z), "+r"(r.w), "+r"(ax));  // drawn before R is looked at
     p.stop = (unsigned long long)ax < J.thr_stop;
-    if (s.R.m) p.x = (int32_t)sample_at(W, s.R.aoff, s.R.m, r);
-  } else {
-    if (s.R.m) p.x = (int32_t)sample_at(W, s.R.aoff, s.R.m, ahead);
+  }
+  if (s.R.m) p.x = (int32_t)sample_at(W, s.R.aoff, s.R.m, r);
+  if (!ppr) {
     ahead = philox(s.i, s.j + 1, 0, J.job, J.k0, J.k1);
     asm volatile("" : "+r"(p.x), "+r"(ahead.x), "+r"(ahead.y), "+r"(ahead.z), "+r"(ahead.w));  // before x is looked at
   }

@@ -212,7 +212,8 @@ int bingo_walk_noalloc(bingo_handle* h, const bingo_walk_job* jobs, uint32_t n_j
  * sees the graph as left by the ops before it. All arrays must be device
  * memory (starts may be NULL). With BINGO_RUN_GRAPH the program is captured
  * once into a CUDA graph and replayed while its shape (op kinds, batch sizes,
- * walk counts per job, array addresses) stays the same; walk-job contents
+ * walk counts per job, array addresses, whether a walk op has node2vec jobs)
+ * stays the same, and captured again when it changes; walk-job contents
  * (apps, lengths, seeds, p/q, stop probabilities) may change between
  * replays. Update capacity is checked on the device: a batch that does not
  * fit the graph arenas is not applied and the call returns
