@@ -636,16 +636,20 @@ __global__ void __launch_bounds__(kBlock, walk_min_blocks(APP))
   // Steps so far; the last claim's size and step; walks claimed.
   uint32_t turn = 0, claim = kClaimMin, claimed = 0, taken = 0;
   const uint32_t warps = gridDim.x * (kBlock / 32);
-  // A small launch's walks spread over all its warps (walks that take trials
-  // spread inside theirs).
-  const uint32_t lanes = kTrials ? 32u : min(32u, walk_share(total, warps));
+  // A small launch's walks spread over all its warps. (Tables with trials keep
+  // to small claims instead, so that every warp has walks of several jobs.)
+  const uint32_t lanes = kTrials && MULTI ? 32u : min(32u, walk_share(total, warps));
   for (;;) {
     uint32_t idle = drained ? 0u : __ballot_sync(kFull, !active);
     uint32_t room = 0;
     if (idle) room = lanes - min(lanes, 32u - __popc(idle));
     while (idle && room && !drained) {
       if (wb >= we) {
-        const uint32_t c = APP >= 0 || chunk ? chunk : taken >= 32 ? next_claim(claim, turn - claimed) : kClaimMin;
+        uint32_t c = chunk;
+        if (APP < 0 && !chunk) c = taken >= 32 ? next_claim(claim, turn - claimed) : kClaimMin;
+        // node2vec's first fill is one claim: eight of 4 from the one counter
+        // took 250,000 walks x 20 on R-MAT 16 from 132 us to 153.
+        if (kTrials && !MULTI && !taken && lanes == 32) c = 32;
         claim = c, claimed = turn, taken += c;
         unsigned long long base = 0;
         if (lane == 0) base = min(atomicAdd(&queue->next, (unsigned long long)c), (unsigned long long)total);
@@ -734,8 +738,9 @@ unsigned walk_blocks_per_sm() {
 // all apps on R-MAT 20 (1.1 M walks) took 3.3 ms at 32 walks per claim, 2.2
 // at 8 and 1.95 at 4; DeepWalk (1 M walks) 1080 us at 8, 1093 at 16; node2vec
 // 4. Mixed tables (0) fit their claims to the walks they meet (next_claim). A
-// launch that fits its lanes claims each warp's share at once. One-hop sampling
-// (one step per item) keeps the occupancy limit and 32.
+// launch that fits its lanes claims each warp's share at once (150,000 node2vec
+// walks x 20, p = q = 1, R-MAT 16: 68 us; in claims of 4, 112). One-hop
+// sampling (one step per item) keeps the occupancy limit and 32.
 constexpr unsigned walk_default_bps(int app) { return app == APP_SAMPLING || walk_trials(app) ? 0 : 4; }
 constexpr uint32_t walk_default_chunk(int app) { return app < 0 ? 0 : app == APP_NODE2VEC ? 4 : app == APP_DEEPWALK ? 8 : 32; }
 
@@ -745,10 +750,10 @@ unsigned walk_bps(unsigned occ, const Tuning& t, int app) {
   const unsigned want = t.walk_blocks_per_sm ? t.walk_blocks_per_sm : walk_default_bps(app);
   return want ? std::max(1u, std::min(occ, want)) : occ;
 }
-uint32_t walk_chunk_of(const Tuning& t, int app, uint32_t total, unsigned grid) {
+uint32_t walk_chunk_of(const Tuning& t, int app, bool multi, uint32_t total, unsigned grid) {
   if (t.walk_chunk) return t.walk_chunk;
   const uint32_t warps = grid * (kBlock / 32);
-  const bool one_fill = !walk_trials(app) && total <= 32ull * warps;  // every warp claims its share at once
+  const bool one_fill = !(walk_trials(app) && multi) && total <= 32ull * warps;  // every warp claims its share at once
   return one_fill ? walk_share(total, warps) : walk_default_chunk(app);
 }
 
@@ -767,7 +772,7 @@ void launch_walk(cudaStream_t st, const WalkView& W, const WalkJobDev& J0, const
                  const uint32_t* prefix, uint32_t n_jobs, uint32_t total, WalkQueue* queue, const Tuning& t) {
   const unsigned grid = walk_grid<APP, MULTI>(total, t);
   k_walk<APP, MULTI><<<grid, kBlock, 0, st>>>(W, J0, jobs, prefix, n_jobs, total, queue,
-                                              walk_chunk_of(t, APP, total, grid));
+                                              walk_chunk_of(t, APP, MULTI, total, grid));
 }
 
 // Launches the persistent walk kernel for a device job table whose jobs all

@@ -351,10 +351,11 @@ __device__ __forceinline__ Proposal warp_propose(const WalkView& W, const WalkJo
   if (ret) hash_peek(rp, W.hash + R.hoff, R.hmask, (uint32_t)s.prev);
   constexpr uint32_t kNone = 0xffffffffu;
   uint32_t won = kNone, probed = 0;  // the accepted trial; this lane's trials that looked up the adjacency index
-  if (APP < 0 && !__any_sync(kFull, n > 1)) {
-    // A draw per lane at most (DeepWalk, PPR, q <= 1), as in many warps of a
-    // mixed table: each draws its own. (A table of node2vec alone seldom gets
-    // here: 1952 us without, 1958 with.)
+  if (!__any_sync(kFull, n > 1)) {
+    // A draw per lane at most (DeepWalk, PPR, q <= 1): each draws its own.
+    // R-MAT 16, p = q = 1, 4,000 walks x 80: 143 us listed, 114 so; p = q =
+    // 0.25: 257 and 220. (Walks with q > 1 seldom get here: 1 M walks x 40 on
+    // R-MAT 20 take 1952 us without this and 1958 with it.)
     if (n) {
       const Trial r = draw_trial(W, J, s.i, s.j, s.t, R.aoff, R.m, n2v, n2v ? sc.ax[mine] : 0u, s.prev, s.phoff, s.phmask);
       if (r.ok) won = 0, p.x = r.x;
