@@ -757,20 +757,32 @@ uint32_t walk_chunk_of(const Tuning& t, int app, bool multi, uint32_t total, uns
   return one_fill ? walk_share(total, warps) : walk_default_chunk(app);
 }
 
-// Blocks of a walk launch: one resident wave at most, and at least
-// walk_per_block walks per block: half-full warps on twice the SMs finish
-// sooner (16,384 DeepWalk walks of 80 on R-MAT 14: 80 us at 256 walks per
-// block, 73 at 128), and walks that take trials use the idle lanes.
-constexpr unsigned walk_per_block(int app) { return walk_trials(app) ? 64 : app == APP_SAMPLING ? 256 : 128; }
-template <int APP, bool MULTI>
-unsigned walk_grid(unsigned long long total, const Tuning& t) {
-  return grid_for(total, walk_per_block(APP), walk_bps(walk_blocks_per_sm<APP, MULTI>(), t, APP));
+// Blocks of a walk launch: one resident wave at most. Where steps list trials
+// (mixed tables, node2vec with q > 1) the idle lanes of a warp serve its other
+// walks, so a small launch takes a block per 64 walks. Else half-full warps on
+// twice the SMs finish sooner (16,384 DeepWalk walks x 80 on R-MAT 14: 80 us at
+// 256 walks per block, 73 at 128), but only as long as SMs would be idle
+// otherwise: past two blocks per SM they only issue more instructions (65,536
+// walks: 118 us at 128 walks per block, 84 so; PPR with stop 0.0125 147 and 92;
+// on R-MAT 20 200 and 185, 183 and 176; node2vec with p = q = 1 204 and 143).
+// Past that, as many on every SM: 586 blocks took 150,000 walks from 134 us
+// (592) to 177, and 100,003 PPR walks on R-MAT 19 take 218 us at 444, 224 at 391
+// and 227 at 592.
+bool spreads_trials(int app, bool multi, const WalkJobDev& J0) {
+  return app == APP_MIXED || (app == APP_NODE2VEC && (multi || J0.thr_out < (1ull << 32)));
+}
+unsigned walk_grid(int app, bool multi, const WalkJobDev& J0, unsigned long long total, unsigned bps) {
+  if (spreads_trials(app, multi, J0)) return grid_for(total, 64, bps);
+  const unsigned long long sms = sm_count(), full = (total + kBlock - 1) / kBlock, half = (total + 127) / 128;
+  unsigned long long blocks = full;
+  if (app != APP_SAMPLING) blocks = full <= 2 * sms ? std::max(full, std::min(half, 2 * sms)) : (full + sms - 1) / sms * sms;
+  return grid_for(blocks, 1, bps);
 }
 
 template <int APP, bool MULTI>
 void launch_walk(cudaStream_t st, const WalkView& W, const WalkJobDev& J0, const WalkJobDev* jobs,
                  const uint32_t* prefix, uint32_t n_jobs, uint32_t total, WalkQueue* queue, const Tuning& t) {
-  const unsigned grid = walk_grid<APP, MULTI>(total, t);
+  const unsigned grid = walk_grid(APP, MULTI, J0, total, walk_bps(walk_blocks_per_sm<APP, MULTI>(), t, APP));
   k_walk<APP, MULTI><<<grid, kBlock, 0, st>>>(W, J0, jobs, prefix, n_jobs, total, queue,
                                               walk_chunk_of(t, APP, MULTI, total, grid));
 }
