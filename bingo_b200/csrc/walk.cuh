@@ -66,8 +66,7 @@ __device__ __forceinline__ VertexRec load_vrec(const WalkView& W, uint32_t u) {
 // Weighted neighbour draw at a vertex with m > 0 alias slots from aoff: slot =
 // mulhi(x, m), r = mulhi64(y:z, T), group = r < thr ? own : alias, member =
 // mulhi(w, cnt) (a one-member group carries its member in the slot:
-// mulhi(w, 1) = 0). In three parts, so that a lane can have several draws'
-// reads in flight.
+// mulhi(w, 1) = 0).
 struct SlotRead {
   unsigned long long thr, T, own_rc, alt_rc;
 };
@@ -276,8 +275,8 @@ __device__ __forceinline__ Proposal walk_propose(const WalkView& W, const WalkJo
 // warp. First-order walks of a mixed table list their one draw, so that all
 // lanes of a mixed warp read together. Bound: random DRAM reads (the
 // adjacency lookups above all). R-MAT 20, 1 M walks x 40, p = 0.5, q = 2:
-// 2550 us with up to three trials in turn per lane, 1979 us; 16 mixed jobs
-// (1.1 M walks, up to 173 steps, q up to 4): 3960 and 1845 us.
+// 2546 us with up to three trials in turn per lane, 1933 so; 16 mixed jobs
+// (1.1 M walks, up to 173 steps, q up to 4): 3986 and 1672 us.
 constexpr uint32_t kTrialItems = 128;  // trials a warp lists per step
 constexpr uint32_t kTrialMax = 16;     // trials a lane lists per step at most
 
